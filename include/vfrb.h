@@ -180,8 +180,10 @@ int vfrb_ddplan_max_delay(const vfrb_ddplan* plan);
  * staged/direct kernels apply (no reference counterpart; introspection). */
 int vfrb_ddplan_group_size(const vfrb_ddplan* plan);
 
-/* Kernel variants of the dedisperser (no reference counterpart).  AUTO uses
- * the autotuned choice (or the largest register group that fits). */
+/* Kernel variants of the dedisperser (no reference counterpart).  AUTO runs
+ * the band-wise kernel for eight or more (nearly) equally spaced trials, else
+ * the autotuned choice (or the largest register group that fits); an explicit
+ * variant runs that kernel. */
 #define VFRB_DD_AUTO 0
 #define VFRB_DD_STAGED 1   /* shared-memory tile, one load per add           */
 #define VFRB_DD_REG1 2     /* register window, 1 trial per thread            */
@@ -194,7 +196,8 @@ int vfrb_ddplan_group_size(const vfrb_ddplan* plan);
 int vfrb_ddplan_set_variant(vfrb_ddplan* plan, int storage, int variant);
 int vfrb_ddplan_variant(const vfrb_ddplan* plan, int storage);
 /* Times every applicable variant on scratch data of the given shape
- * (nt_out samples per trial, `storage` form) and keeps the fastest.  Writes
+ * (nt_out samples per trial, `storage` form) and keeps the fastest for calls
+ * that the band-wise kernel does not take (see VFRB_DD_AUTO).  Writes
  * the per-variant times in ms to times[VFRB_DD_NVARIANTS] (index = variant,
  * < 0 = not applicable).  FP16 variants are timed without a shifted ring
  * (vfrb_dd_args.fb_shift1); given one, VFRB_DD_PAT4 runs its faster pair
@@ -227,7 +230,8 @@ typedef struct vfrb_dd_args {
                               * `fb` shifted by one row (fb_shift1[c][r] =
                               * fb[c][r + 1] for every row but the last valid
                               * one; vfrb_bp_args.out_shift1 writes it).  The
-                              * four-trial pattern kernel then reads windows of
+                              * four-trial pattern kernel (VFRB_DD_PAT4; the
+                              * band-wise kernel needs no copy) reads windows of
                               * halves with 4-byte loads; results equal the
                               * plain FP16 form's up to FP32 summation order */
 } vfrb_dd_args;

@@ -1,0 +1,246 @@
+// Tables of the band-wise dedispersion kernel (dedisperse_band.cu), built on the
+// host from a delay table when a plan is created.  Plain C++.
+#pragma once
+#include <algorithm>
+#include <climits>
+#include <cmath>
+#include <cstdint>
+#include <vector>
+
+namespace vfrb {
+
+constexpr int kBandD = 8;                 // trials per group
+constexpr int kBandW = 16;                // warps per CTA, one CTA per SM
+constexpr int kBandSmax = 4;              // most rows that a group's shifts span
+constexpr int kBandAlign = 16;            // rows: tile starts of every storage form are 16-byte aligned
+constexpr int kBandNtMax = 320;           // longest tile (FP16): the row length in shared memory is common to all forms
+constexpr int kBandSmem = 220 * 1024;     // that the tables plan for
+constexpr int kBandSmemMax = 227 * 1024;  // a CTA's limit
+constexpr int kBandMaxCh = 96;
+constexpr int kBandMax = 64;              // bands
+constexpr int kBandGeneric = 256;         // pattern code of shifts that are no staircase
+
+struct BandDesc {
+  int c_lo, nch;    // channels [c_lo, c_lo + nch)
+  int m;            // rows per trial taken off
+  int ch, nchunks;  // channels per chunk
+  int lm;           // tile row length in elements
+  int chunk0;       // index of its first chunk among the plan's records
+};
+
+// a group's record of a chunk: slot[ch_cap] (tile offset | channel << 18), run[ch_cap] (code | count << 8), nrun
+constexpr int band_rec_bytes(int ch_cap) { return (ch_cap * 6 + 2 + 15) / 16 * 16; }
+
+struct BandHost {
+  int ndm = 0, nchan = 0, ngroups = 0, nblocks = 0;
+  // Groups per CTA.  Its kBandW warps are `split` sets of them: with fewer
+  // groups each chunk's channels are divided among the sets, whose sums are
+  // added at the end, so a plan of few trials still has CTAs for every SM.  It
+  // depends on the trials alone: the order of the sums must not change with the
+  // number of samples.  (201 trials x 5145 samples: 16 groups per CTA give 44 CTAs
+  // and 1.49 ms, 4 groups 154 CTAs and 0.94 ms.)
+  int gper = kBandW, split = 1;
+  std::vector<BandDesc> bands;
+  std::vector<int> skmin, skmax;   // [band][block] skews of the block's first and last trial
+  int rec_bytes = 0, ch_cap = 0;
+  std::vector<int> bmin;           // [block][nchan] first staged row of the channel, relative to row0 + t'
+  std::vector<int> skew;           // [band][nblocks * gper] skew of each group's first trial
+  std::vector<unsigned char> rec;  // [chunk][nblocks][split][gper][rec_bytes]
+  std::vector<unsigned> shift;     // [group][nchan] eight shifts, 4 bits each; empty when all are staircases
+};
+
+inline long long floor_div(long long a, long long b) { return a >= 0 ? a / b : -((-a + b - 1) / b); }
+inline int floor_to(int a, int b) { return (int)floor_div(a, b) * b; }
+
+// Code of eight shifts that go up (or down) by 0 or 1 from trial to trial:
+// bit q = the step after the q-th trial, counted from the trial with shift 0;
+// bit 7 = the shifts fall (the count starts at the last trial).
+inline int band_code(const int* sh) {
+  for (int dir = 0; dir < 2; ++dir) {
+    int code = dir << 7, at = 0, q = 0;
+    for (; q < kBandD; ++q) {
+      const int v = sh[dir ? kBandD - 1 - q : q];
+      if (q && v == at + 1) code |= 1 << (q - 1);
+      else if (v != at) break;
+      at = v;
+    }
+    if (q == kBandD) return code;
+  }
+  return kBandGeneric;
+}
+
+// False when the kernel does not apply to the delay table: fewer than eight
+// trials, or trials that are not close to equally spaced.
+inline bool band_build(BandHost& h, const int32_t* off, int ndm, int nchan) {
+  if (ndm < kBandD) return false;
+  BandHost* t = &h;
+  const int D = kBandD;
+  t->ndm = ndm;
+  t->nchan = nchan;
+  const int ng = t->ngroups = (ndm + D - 1) / D;
+  const int G = t->gper = ng <= 40 ? 4 : ng <= 80 ? 8 : 16;
+  const int SP = t->split = kBandW / G;
+  const int nb = t->nblocks = (ng + G - 1) / G;
+  auto start = [&](int g) { return std::min(g * D, ndm - D); };
+  auto row = [&](int d) { return off + (long long)d * nchan; };
+  // bands: runs of channels whose mean delay step per trial rounds to one number
+  std::vector<long long> step(nchan, 0);
+  for (int g = 0; g < ng; ++g) {
+    const int32_t *a = row(start(g)), *z = row(start(g) + D - 1);
+    for (int c = 0; c < nchan; ++c) step[c] += z[c] - a[c];
+  }
+  // (the mean over a few dozen neighbouring channels: whole-number delays make a single channel's noisy)
+  const double per = 1.0 / ((double)ng * (D - 1));
+  std::vector<long long> cum(nchan + 1, 0);
+  for (int c = 0; c < nchan; ++c) cum[c + 1] = cum[c] + step[c];
+  int m = 0;
+  for (int c = 0; c < nchan; ++c) {
+    const int w = std::min(std::min(c, nchan - 1 - c), nchan / 256);
+    const double y = (double)(cum[c + w + 1] - cum[c - w]) * per / (2 * w + 1);
+    if (c == 0 || y > m + 0.51 || y < m - 0.51) {
+      const int mn = (int)std::lrint(y);
+      if (c == 0 || mn != m) {
+        if ((int)t->bands.size() == kBandMax || mn > 4096 || mn < -4096) return false;
+        m = mn;
+        BandDesc b{};
+        b.c_lo = c;
+        b.m = m;
+        t->bands.push_back(b);
+      }
+    }
+    ++t->bands.back().nch;
+  }
+  const int nbands = (int)t->bands.size();
+  // per (group, channel): window start relative to row0 + t', pattern, shifts
+  std::vector<int> base((size_t)ng * nchan);
+  std::vector<unsigned short> pat((size_t)ng * nchan);
+  std::vector<unsigned>& shift = t->shift;
+  std::vector<int>& skew = t->skew;
+  skew.assign((size_t)nbands * nb * G, 0);
+  for (int bi = 0; bi < nbands; ++bi) {
+    const BandDesc& b = t->bands[bi];
+    const int mid = b.c_lo + b.nch / 2;
+    for (int g = 0; g < ng; ++g) {
+      const int gs = start(g);
+      const int sk = row(gs)[mid];
+      skew[(size_t)bi * nb * G + g] = sk;
+      const int32_t* r[D];
+      for (int j = 0; j < D; ++j) r[j] = row(gs + j);
+      for (int c = b.c_lo; c < b.c_lo + b.nch; ++c) {
+        int v[D], mn = 0x7fffffff, mx = -0x7fffffff;
+        for (int j = 0; j < D; ++j) {
+          v[j] = r[j][c] - j * b.m;
+          mn = std::min(mn, v[j]);
+          mx = std::max(mx, v[j]);
+        }
+        if (mx - mn > kBandSmax) return false;  // not (nearly) equally spaced
+        for (int j = 0; j < D; ++j) v[j] -= mn;
+        const size_t i = (size_t)g * nchan + c;
+        base[i] = mn - sk;
+        pat[i] = (unsigned short)band_code(v);
+        if (pat[i] == kBandGeneric) {
+          if (shift.empty()) shift.assign((size_t)ng * nchan, 0u);
+          unsigned s = 0;
+          for (int j = 0; j < D; ++j) s |= (unsigned)v[j] << (4 * j);
+          shift[i] = s;
+        }
+      }
+    }
+  }
+  size_t ngen = 0;
+  if (!shift.empty())
+    for (unsigned short q : pat) ngen += q == kBandGeneric;
+  if (ngen * 20 > pat.size()) return false;  // more than 5% off the staircases: the other kernels are faster
+  // per block: first staged row of each channel, and the tile row length of each band
+  std::vector<int>& bmin = t->bmin;
+  bmin.assign((size_t)nb * nchan, 0);
+  std::vector<int> span(nbands, 0);
+  for (int bi = 0; bi < nbands; ++bi)
+    for (int c = t->bands[bi].c_lo; c < t->bands[bi].c_lo + t->bands[bi].nch; ++c)
+      for (int k = 0; k < nb; ++k) {
+        int mn = 0x7fffffff, mx = -0x7fffffff;
+        for (int g = k * G; g < std::min(ng, (k + 1) * G); ++g) {
+          mn = std::min(mn, base[(size_t)g * nchan + c]);
+          mx = std::max(mx, base[(size_t)g * nchan + c]);
+        }
+        mn = floor_to(mn, kBandAlign);
+        bmin[(size_t)k * nchan + c] = mn;
+        span[bi] = std::max(span[bi], mx - mn);
+      }
+  int chunk0 = 0, cap = 1;
+  for (int bi = 0; bi < nbands; ++bi) {
+    BandDesc& b = t->bands[bi];
+    b.lm = (kBandAlign - 1 + span[bi] + kBandNtMax + kBandSmax + 1 + kBandAlign - 1) / kBandAlign * kBandAlign;
+    // two buffers of FP32 rows and records
+    int ch = (kBandSmem - 64) / (2 * (b.lm * 4 + 6 * kBandW + 4) + 64);
+    ch = std::min(ch, kBandMaxCh);
+    ch = std::min(ch, 32 * kBandW);
+    if (ch < 8) return false;  // the block's trials spread too far to share staged rows
+    b.nchunks = (b.nch + ch - 1) / ch;
+    b.ch = (b.nch + b.nchunks - 1) / b.nchunks;  // even chunks
+    b.chunk0 = chunk0;
+    chunk0 += b.nchunks;
+    cap = std::max(cap, (b.ch + SP - 1) / SP);
+  }
+  cap = (cap + 2) & ~1;  // and a slot of padding, read ahead
+  t->ch_cap = cap;
+  t->rec_bytes = band_rec_bytes(cap);
+  const size_t ngp = (size_t)nb * G;
+  std::vector<unsigned char>& rec = t->rec;
+  rec.assign((size_t)chunk0 * nb * kBandW * t->rec_bytes, 0);
+  for (int bi = 0; bi < nbands; ++bi) {
+    const BandDesc& b = t->bands[bi];
+    for (int k = 0; k < b.nchunks; ++k)
+      for (int g = 0; g < ng; ++g) {
+        const int c0 = b.c_lo + k * b.ch, nc = std::min(b.ch, b.nch - k * b.ch);
+        const unsigned short* pp = &pat[(size_t)g * nchan + c0];
+        int cnt[257] = {0}, pos[257], n = 0;
+        unsigned char ord[kBandMaxCh];
+        for (int i = 0; i < nc; ++i) ++cnt[pp[i]];
+        for (int i = 0; i < 257; ++i) {
+          pos[i] = n;
+          n += cnt[i];
+        }
+        for (int i = 0; i < nc; ++i) ord[pos[pp[i]]++] = (unsigned char)i;
+        for (int sp = 0; sp < SP; ++sp) {  // this set's share of the sorted channels
+          unsigned char* q =
+              rec.data() + (((size_t)(b.chunk0 + k) * nb + g / G) * kBandW + sp * G + g % G) * t->rec_bytes;
+          unsigned* slot = reinterpret_cast<unsigned*>(q);
+          unsigned short* run = reinterpret_cast<unsigned short*>(q + 4 * cap);
+          int nrun = 0, last = -1;
+          const int lo = nc * sp / SP, hi = nc * (sp + 1) / SP;
+          for (int i = lo; i < hi; ++i) {
+            const int cl = ord[i], code = pp[cl];
+            const int rel = base[(size_t)g * nchan + c0 + cl] - bmin[(size_t)(g / G) * nchan + c0 + cl];
+            slot[i - lo] = (unsigned)(cl * b.lm + rel) | ((unsigned)cl << 18);
+            if (code == kBandGeneric) run[nrun++] = 0;  // no count: one channel with its own shifts
+            else if (code == last) run[nrun - 1] += 1 << 8;
+            else run[nrun++] = (unsigned short)(code | (1 << 8));
+            last = code;
+          }
+          run[cap] = (unsigned short)nrun;
+        }
+      }
+  }
+  // skews of a block's first and last trial, per band (launch geometry)
+  t->skmin.resize((size_t)nbands * nb);
+  t->skmax.resize((size_t)nbands * nb);
+  for (int bi = 0; bi < nbands; ++bi)
+    for (int k = 0; k < nb; ++k) {
+      int mn = 0x7fffffff, mx = -0x7fffffff;
+      for (int g = k * G; g < std::min(ng, (k + 1) * G); ++g)
+        for (int j = 0; j < D; j += D - 1) {
+          mn = std::min(mn, skew[(size_t)bi * ngp + g] + j * t->bands[bi].m);
+          mx = std::max(mx, skew[(size_t)bi * ngp + g] + j * t->bands[bi].m);
+        }
+      t->skmin[(size_t)bi * nb + k] = mn;
+      t->skmax[(size_t)bi * nb + k] = mx;
+      // the kernel takes them from the first and the last group (delays grow with the trial)
+      const int g0 = k * G, g1 = std::min(ng, (k + 1) * G) - 1;
+      if (mn != skew[(size_t)bi * ngp + g0] || mx != skew[(size_t)bi * ngp + g1] + (D - 1) * t->bands[bi].m)
+        return false;
+    }
+  return true;
+}
+
+}  // namespace vfrb

@@ -13,6 +13,7 @@
 // memory read of a warp is 32 consecutive elements (conflict free) and the
 // per-channel delay is warp-uniform.  Accumulation is FP32 in registers; the
 // FP16 / int8 forms apply the per-channel weight with an FMA.
+#include "dedisp_band.h"
 #include "vfrb_common.cuh"
 
 #include <algorithm>
@@ -317,6 +318,57 @@ __global__ void __launch_bounds__(256) k_series_stats(const float* __restrict__ 
   dm_finalize(d, nt, s, s2, mx, arg, ave, sigma, peak, frb, argmax);
 }
 
+// calcstats partials of whole series: one CTA per (DM, kPartNt samples).
+constexpr int kPartNt = 2048;
+__global__ void __launch_bounds__(256) k_series_part(const float* __restrict__ dd, long long nt, long long stride,
+                                                     int ndm, int ntb, DmPartial* __restrict__ part) {
+  const int tb = (int)(blockIdx.x % (unsigned)ntb), d = (int)(blockIdx.x / (unsigned)ntb);
+  const float* x = dd + (long long)d * stride;
+  const long long t0 = (long long)tb * kPartNt + threadIdx.x;
+  float v[kPartNt / 256];
+#pragma unroll
+  for (int i = 0; i < kPartNt / 256; ++i) v[i] = t0 + 256 * i < nt ? x[t0 + 256 * i] : 0.f;
+  double s = 0.0, s2 = 0.0;
+  float mx = -INFINITY;
+  int arg = 0x7fffffff;
+#pragma unroll
+  for (int i = 0; i < kPartNt / 256; ++i) {
+    if (t0 + 256 * i < nt) {
+      s += (double)v[i];
+      s2 += (double)v[i] * (double)v[i];
+      if (v[i] > mx) {  // t grows: the first maximum is kept
+        mx = v[i];
+        arg = (int)(t0 + 256 * i);
+      }
+    }
+  }
+  __shared__ DmPartial red[8];
+  s = wsum(s);
+  s2 = wsum(s2);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const float omx = __shfl_xor_sync(0xffffffffu, mx, o);
+    const int oarg = __shfl_xor_sync(0xffffffffu, arg, o);
+    if (omx > mx || (omx == mx && oarg < arg)) {
+      mx = omx;
+      arg = oarg;
+    }
+  }
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = DmPartial{s, s2, mx, arg};
+  __syncthreads();
+  if (threadIdx.x != 0) return;
+  DmPartial q = red[0];
+  for (int w = 1; w < 8; ++w) {
+    q.s += red[w].s;
+    q.s2 += red[w].s2;
+    if (red[w].mx > q.mx || (red[w].mx == q.mx && red[w].arg < q.arg)) {
+      q.mx = red[w].mx;
+      q.arg = red[w].arg;
+    }
+  }
+  part[(long long)tb * ndm + d] = q;
+}
+
 int launch_series_stats(const float* dd, int ndm, long long nt, long long stride, float* ave, float* sigma,
                         float* peak, int* frb, int* argmax, cudaStream_t s) {
   if (!dd || ndm < 1 || nt < 2 || stride < nt || nt > 0x7fffffffLL) return VFRB_ERR_ARG;
@@ -430,8 +482,14 @@ struct vfrb_ddplan {
   int max_delay = 0;  // max over the table
   int span16 = 0;     // max over 16-trial blocks and channels of (max - min) delay
   int* d_off = nullptr;
-  vfrb::RegGroup reg[3];            // D = 4, 2, 1 when applicable
+  vfrb::RegGroup reg[3];            // D = 4, 2, 1 when applicable (see ddplan_groups)
+  bool group_ok[5] = {};            // [D]: the groups of D trials apply
+  bool groups_built = false;
   int variant[3] = {0, 0, 0};       // chosen variant per storage form (VFRB_DD_*)
+  // AUTO runs the band kernel where it applies (dedisperse_band.cu), else the
+  // fastest of the others when they have been timed, else the default
+  int tuned[3] = {0, 0, 0};
+  vfrb::BandTables* band = nullptr;
 };
 
 namespace vfrb {
@@ -649,21 +707,34 @@ static int pat_launch(const vfrb_ddplan* pl, int v, const vfrb_dd_args& a, DmPar
 
 static int default_variant(const vfrb_ddplan* pl, int storage) {
   if (storage == VFRB_F32 || storage == VFRB_F16) {
-    const RegGroup* g4 = find_group(pl, 4);
-    const RegGroup* g2 = find_group(pl, 2);
-    if (g4 && g4->d_gpat) return VFRB_DD_PAT4;
-    if (g2 && g2->d_gpat) return VFRB_DD_PAT2;
-  }
-  if (storage == VFRB_F32) {
-    if (find_group(pl, 4)) return VFRB_DD_REG4;
-    if (find_group(pl, 2)) return VFRB_DD_REG2;
-    if (find_group(pl, 1)) return VFRB_DD_REG1;
-  } else if (storage == VFRB_F16) {
-    if (find_group(pl, 2)) return VFRB_DD_REG2;
-    if (find_group(pl, 4)) return VFRB_DD_REG4;
-    if (find_group(pl, 1)) return VFRB_DD_REG1;
+    // (the limits on a group's delays are those of the pattern tables)
+    if (pl->group_ok[4]) return VFRB_DD_PAT4;
+    if (pl->group_ok[2]) return VFRB_DD_PAT2;
+    return VFRB_DD_REG1;
   }
   return VFRB_DD_STAGED;
+}
+
+static int resolve_auto(const vfrb_ddplan* pl, int storage) {
+  if (pl->variant[storage] != VFRB_DD_AUTO) return pl->variant[storage];
+  return pl->tuned[storage] != VFRB_DD_AUTO ? pl->tuned[storage] : default_variant(pl, storage);
+}
+
+// The band kernel for this call, with the statistics from the finished
+// series; *launched = 0 when it does not apply.
+static int launch_band(const vfrb_ddplan* pl, const vfrb_dd_args& a, cudaStream_t s, int* launched) {
+  *launched = 0;
+  if (!pl->band || a.sigma_out) return VFRB_OK;
+  const bool want_stats = a.ave || a.sigma || a.peak || a.frb || a.argmax;
+  const long long ntb = (a.nt_out + kPartNt - 1) / kPartNt;
+  if (want_stats && ntb * pl->ndm > 0x7fffffffLL) return VFRB_OK;
+  const int st = band_launch(pl->band, a, nullptr, 0, s, launched);
+  if (st || !*launched || !want_stats) return st;
+  DmPartial* part = reinterpret_cast<DmPartial*>(a.workspace);
+  k_series_part<<<(unsigned)(ntb * pl->ndm), 256, 0, s>>>(a.out, a.nt_out, a.out_stride, pl->ndm, (int)ntb, part);
+  k_dm_stats<<<(pl->ndm + 7) / 8, 256, 0, s>>>(part, (int)ntb, pl->ndm, a.nt_out, a.ave, a.sigma, a.peak, a.frb,
+                                               a.argmax);
+  return cuda_status(cudaGetLastError());
 }
 
 static int launch_variant(const vfrb_ddplan* pl, int v, const vfrb_dd_args& a, cudaStream_t s,
@@ -727,9 +798,12 @@ int launch_dedisperse_plan(const vfrb_ddplan* pl, const vfrb_dd_args& a, cudaStr
   const bool want_stats = a.ave || a.sigma || a.peak || a.frb || a.argmax;
   if (want_stats && (!a.workspace || a.workspace_bytes < dedisperse_workspace_bytes_plan(pl, a.nt_out)))
     return VFRB_ERR_ARG;
-  int v = pl->variant[a.storage];
-  if (v == VFRB_DD_AUTO) v = default_variant(pl, a.storage);
-  return launch_variant(pl, v, a, s, a.fb_shift1);
+  if (pl->variant[a.storage] == VFRB_DD_AUTO) {
+    int launched = 0;
+    const int st = launch_band(pl, a, s, &launched);
+    if (st || launched) return st;
+  }
+  return launch_variant(pl, resolve_auto(pl, a.storage), a, s, a.fb_shift1);
 }
 
 // One launch of the pattern kernel over several streams' chunks (grid z =
@@ -743,9 +817,9 @@ int launch_dedisperse_jobs(const vfrb_ddplan* pl, int storage, const DdJob* jobs
                            unsigned row_mask, cudaStream_t s, int* launched) {
   *launched = 0;
   if (!pl || njobs < 1 || njobs > kDdMaxJobs || storage < VFRB_F32 || storage > VFRB_F16) return VFRB_ERR_ARG;
-  int v = pl->variant[storage];
-  if (v == VFRB_DD_AUTO) v = default_variant(pl, storage);
-  if (v != VFRB_DD_PAT4 && v != VFRB_DD_PAT2) return VFRB_OK;
+  const int v = resolve_auto(pl, storage);
+  const bool band = pl->variant[storage] == VFRB_DD_AUTO && pl->band;
+  if (!band && v != VFRB_DD_PAT4 && v != VFRB_DD_PAT2) return VFRB_OK;
   vfrb_dd_args a{};
   a.fb = jobs[0].fb;
   a.storage = storage;
@@ -765,6 +839,11 @@ int launch_dedisperse_jobs(const vfrb_ddplan* pl, int storage, const DdJob* jobs
   a.nt_out = nt;
   a.out = jobs[0].out;
   a.out_stride = jobs[0].out_stride;
+  if (band) {
+    const int st = band_launch(pl->band, a, jobs, njobs, s, launched);
+    if (st || *launched) return st;
+    if (v != VFRB_DD_PAT4 && v != VFRB_DD_PAT2) return VFRB_OK;
+  }
   int ntb = 0;
   const int st = pat_launch(pl, v, a, nullptr, s, &ntb, jobs, njobs, pair ? jobs[0].fb1 : nullptr);
   if (st) return st;
@@ -772,9 +851,12 @@ int launch_dedisperse_jobs(const vfrb_ddplan* pl, int storage, const DdJob* jobs
   return VFRB_OK;
 }
 
+static int ddplan_groups(vfrb_ddplan* p, const int32_t* h_off);
+
 // Time every applicable variant on scratch data and keep the fastest.
 int ddplan_autotune(vfrb_ddplan* pl, int storage, long long nt, float* times, cudaStream_t s) {
   if (!pl || storage < VFRB_F32 || storage > VFRB_I8 || nt <= 0) return VFRB_ERR_ARG;
+  if (const int st = ddplan_groups(pl, nullptr)) return st;
   const size_t eb = storage == VFRB_F32 ? 4 : storage == VFRB_F16 ? 2 : 1;
   const long long rows = (nt + pl->max_delay + 15) / 16 * 16;
   void* fb = nullptr;
@@ -831,6 +913,12 @@ int ddplan_autotune(vfrb_ddplan* pl, int storage, long long nt, float* times, cu
   }
   float best = 1e30f;
   int bestv = VFRB_DD_STAGED;
+  // The band kernel (AUTO) is kept wherever it applies, not timed: it was the
+  // fastest at every size tried (8 to 2048 trials, 300 to 16,384 samples, 1.4 to
+  // 4.6 times the best of the others), and plans made side by side, whose timings
+  // disturb each other, then sum in the same order.
+  int band = 0;
+  if (launch_band(pl, a, s, &band) != VFRB_OK) band = 0;
   if (times) times[VFRB_DD_AUTO] = -1.f;
   // the direct variant last: it is timed only when nothing faster applies
   static const int order[] = {VFRB_DD_STAGED, VFRB_DD_REG1, VFRB_DD_REG2, VFRB_DD_REG4,
@@ -864,20 +952,25 @@ int ddplan_autotune(vfrb_ddplan* pl, int storage, long long nt, float* times, cu
   const int err = cuda_status(cudaStreamSynchronize(s));
   cleanup();
   if (err) return err;
-  pl->variant[storage] = bestv;
+  pl->tuned[storage] = bestv;
+  pl->variant[storage] = band ? VFRB_DD_AUTO : bestv;
   return VFRB_OK;
 }
 
 int ddplan_set_variant(vfrb_ddplan* pl, int storage, int v) {
   if (!pl || storage < VFRB_F32 || storage > VFRB_I8 || v < VFRB_DD_AUTO || v >= VFRB_DD_NVARIANTS)
     return VFRB_ERR_ARG;
+  if (v != VFRB_DD_AUTO) {
+    const int st = ddplan_groups(pl, nullptr);
+    if (st) return st;
+  }
   pl->variant[storage] = v;
   return VFRB_OK;
 }
 
 int ddplan_variant(const vfrb_ddplan* pl, int storage) {
   if (!pl || storage < VFRB_F32 || storage > VFRB_I8) return -1;
-  return pl->variant[storage] == VFRB_DD_AUTO ? default_variant(pl, storage) : pl->variant[storage];
+  return resolve_auto(pl, storage);
 }
 
 // Pattern id of the packed in-group differences (8 bits per trial, trial 0
@@ -973,7 +1066,7 @@ static int build_group(vfrb_ddplan* p, const int32_t* h_off, int D, int smax_all
   g.nblocks16 = nb16;
   g.span_16w = span16;
   for (int b = 0; b < nb16; ++b) g.bmin_mid_max16 = std::max(g.bmin_mid_max16, bm16[(size_t)b * nchan + nchan / 2]);
-  const bool with_pat = (D == 4 && smax <= VFRB_PAT4_SMAX) || (D == 2 && smax <= VFRB_PAT2_SMAX);
+  const bool with_pat = D == 4 || D == 2;
   std::vector<unsigned char> pt;
   if (with_pat) {
     pt.resize(gp.size());
@@ -1005,9 +1098,35 @@ static int build_group(vfrb_ddplan* p, const int32_t* h_off, int D, int smax_all
   return VFRB_OK;
 }
 
+constexpr int kGroupSmax4 = VFRB_PAT4_SMAX, kGroupSmax2 = VFRB_PAT2_SMAX;
+
+// Tables of the register-window and pattern kernels.  Where the band kernel
+// applies they are built when a variant is chosen or timed (their tables cost as
+// much to make as the rest of the plan): before any launch that uses them, so
+// that no launch allocates.
+static int ddplan_groups(vfrb_ddplan* p, const int32_t* h_off) {
+  if (p->groups_built) return VFRB_OK;
+  std::vector<int32_t> back;
+  if (!h_off) {
+    back.resize((size_t)p->ndm * p->nchan);
+    if (cudaMemcpy(back.data(), p->d_off, back.size() * sizeof(int32_t), cudaMemcpyDeviceToHost) != cudaSuccess) {
+      cudaGetLastError();
+      return VFRB_ERR_CUDA;
+    }
+    h_off = back.data();
+  }
+  int st = VFRB_OK;
+  if (p->group_ok[4]) st = build_group(p, h_off, 4, kGroupSmax4);
+  if (!st && p->group_ok[2]) st = build_group(p, h_off, 2, kGroupSmax2);
+  if (!st && p->group_ok[1]) st = build_group(p, h_off, 1, 0);
+  p->groups_built = st == VFRB_OK;
+  return st;
+}
+
 int ddplan_destroy(vfrb_ddplan* p) {
   if (!p) return VFRB_OK;
   if (p->d_off) cudaFree(p->d_off);
+  band_destroy(p->band);
   for (auto& g : p->reg) {
     if (g.d_gbase) cudaFree(g.d_gbase);
     if (g.d_gpack) cudaFree(g.d_gpack);
@@ -1024,29 +1143,39 @@ int ddplan_create(vfrb_ddplan** out, const int32_t* h_off, int ndm, int nchan) {
   vfrb_ddplan* p = new vfrb_ddplan();
   p->ndm = ndm;
   p->nchan = nchan;
-  int mxd = 0, span = 0;
-  for (long long i = 0; i < (long long)ndm * nchan; ++i) {
-    if (h_off[i] < 0) {
-      delete p;
-      return VFRB_ERR_ARG;
-    }
-    mxd = std::max(mxd, (int)h_off[i]);
-  }
-  for (int d0 = 0; d0 < ndm; d0 += kDdDm)
+  // one pass over the table, four trials at a time: the largest delay, the
+  // largest spread of 16-trial blocks, and of the groups of four and two
+  int least = 0, mxd = 0, span = 0, range4 = 0, range2 = 0;
+  std::vector<int> mn(nchan), mx(nchan);
+  for (int d0 = 0; d0 < ndm; d0 += 4) {
+    const int32_t* r[4];
+    for (int j = 0; j < 4; ++j) r[j] = h_off + (long long)std::min(d0 + j, ndm - 1) * nchan;
+    const bool fresh = d0 % kDdDm == 0;
     for (int c = 0; c < nchan; ++c) {
-      int mn = 0x7fffffff, mx = 0;
-      for (int d = d0; d < std::min(ndm, d0 + kDdDm); ++d) {
-        mn = std::min(mn, (int)h_off[(long long)d * nchan + c]);
-        mx = std::max(mx, (int)h_off[(long long)d * nchan + c]);
-      }
-      span = std::max(span, mx - mn);
+      const int a = r[0][c], b = r[1][c], e = r[2][c], f = r[3][c];
+      const int lo1 = std::min(a, b), hi1 = std::max(a, b), lo2 = std::min(e, f), hi2 = std::max(e, f);
+      const int lo = std::min(lo1, lo2), hi = std::max(hi1, hi2);
+      range2 = std::max(range2, std::max(hi1 - lo1, hi2 - lo2));
+      range4 = std::max(range4, hi - lo);
+      least = std::min(least, lo);
+      mxd = std::max(mxd, hi);
+      mn[c] = fresh ? lo : std::min(mn[c], lo);
+      mx[c] = fresh ? hi : std::max(mx[c], hi);
+      span = std::max(span, mx[c] - mn[c]);
     }
+  }
+  if (least < 0) {
+    delete p;
+    return VFRB_ERR_ARG;
+  }
   p->max_delay = mxd;
   p->span16 = span;
   // register-window groups: D = 4 and 2 when their in-group shifts fit, else D = 1
-  int st = build_group(p, h_off, 4, 20);
-  if (!st) st = build_group(p, h_off, 2, 16);
-  if (!st && !find_group(p, 2) && !find_group(p, 4)) st = build_group(p, h_off, 1, 0);
+  p->group_ok[4] = range4 <= kGroupSmax4;
+  p->group_ok[2] = range2 <= kGroupSmax2;
+  p->group_ok[1] = !p->group_ok[4] && !p->group_ok[2];
+  int st = band_create(&p->band, h_off, ndm, nchan);
+  if (!st && !p->band) st = ddplan_groups(p, h_off);
   if (st) {
     ddplan_destroy(p);
     return st;
