@@ -181,9 +181,9 @@ int vfrb_ddplan_max_delay(const vfrb_ddplan* plan);
 int vfrb_ddplan_group_size(const vfrb_ddplan* plan);
 
 /* Kernel variants of the dedisperser (no reference counterpart).  AUTO runs
- * the band-wise kernel for eight or more (nearly) equally spaced trials, else
- * the autotuned choice (or the largest register group that fits); an explicit
- * variant runs that kernel. */
+ * a streaming kernel for few trials and the band-wise kernel for (nearly)
+ * equally spaced trials, else the autotuned choice (or the largest register
+ * group that fits); an explicit variant runs that kernel. */
 #define VFRB_DD_AUTO 0
 #define VFRB_DD_STAGED 1   /* shared-memory tile, one load per add           */
 #define VFRB_DD_REG1 2     /* register window, 1 trial per thread            */
@@ -197,7 +197,7 @@ int vfrb_ddplan_set_variant(vfrb_ddplan* plan, int storage, int variant);
 int vfrb_ddplan_variant(const vfrb_ddplan* plan, int storage);
 /* Times every applicable variant on scratch data of the given shape
  * (nt_out samples per trial, `storage` form) and keeps the fastest for calls
- * that the band-wise kernel does not take (see VFRB_DD_AUTO).  Writes
+ * that neither of AUTO's own kernels takes (see VFRB_DD_AUTO).  Writes
  * the per-variant times in ms to times[VFRB_DD_NVARIANTS] (index = variant,
  * < 0 = not applicable).  FP16 variants are timed without a shifted ring
  * (vfrb_dd_args.fb_shift1); given one, VFRB_DD_PAT4 runs its faster pair

@@ -1,5 +1,5 @@
-"""The band-wise dedispersion kernel (the automatic choice for equally spaced
-trials) against the FP64 oracle: every storage form with and without channel
+"""The automatic choice's own dedispersion kernels -- streaming for few trials,
+band-wise for equally spaced ones -- against the FP64 oracle: every storage form with and without channel
 weights, sizes at the edges of its tiles and trial groups, ring wrap, rows
 outside the valid ones (NaN there must not reach an output), batched statistics.
 
@@ -35,7 +35,9 @@ def _case(ndm, nch, nt, dm_max, seed, storage, row0, R):
 
 @pytest.mark.parametrize("storage,weighted", [(0, False), (1, False), (1, True), (2, False), (2, True)])
 @pytest.mark.parametrize("ndm,nch,nt,dm_max,row0,R", [
-    (8, 64, 1, 3.0, 0, 0),            # one group, one sample
+    (1, 64, 1, 3.0, 0, 0),            # streaming: one trial, one sample
+    (16, 333, 1290, 40.0, 900, 2048), # streaming: most trials, a ragged channel count, the ring wraps
+    (17, 64, 1, 3.0, 0, 0),           # one sample; the last group overlaps the one before
     (50, 320, 449, 30.0, 0, 0),       # last group overlaps the one before; one past an FP16 tile
     (97, 256, 1500, 90.0, 5, 0),      # a start off the alignment
     (33, 512, 960, 8.0, 1900, 2048),  # the ring wraps
@@ -43,7 +45,7 @@ def _case(ndm, nch, nt, dm_max, seed, storage, row0, R):
     (400, 128, 289, 60.0, 3, 0),      # eight groups to a CTA
     (700, 64, 700, 40.0, 0, 0),       # sixteen groups to a CTA
 ])
-def test_band_kernel_matches_fp64(vf, O, ndm, nch, nt, dm_max, row0, R, storage, weighted):
+def test_automatic_kernels_match_fp64(vf, O, ndm, nch, nt, dm_max, row0, R, storage, weighted):
     import torch
     off, ring, fb, rows = _case(ndm, nch, nt, dm_max, ndm + nt, storage, row0, R)
     w = np.random.default_rng(5).uniform(0.5, 2.0, nch).astype(np.float32) if weighted else None
@@ -99,3 +101,22 @@ def test_band_kernel_is_the_automatic_choice_and_agrees_with_the_others(vf, O):
         if 0 <= t < 1500:
             want[d, t] = True
     assert np.array_equal(hit, want) and bool(torch.isfinite(got[~torch.from_numpy(want).cuda()]).all())
+
+
+@pytest.mark.parametrize("ndm,nt,row0", [(1, 33, 0), (2, 5000, 1800), (64, 700, 7), (65, 300, 0)])
+def test_sigma_form_sizes(vf, O, ndm, nt, row0):
+    """Sigma form at the sizes where its kernel or samples per lane change, off
+    the alignment and across the ring's end: mean <= 1e-5 of the rms, sigma <=
+    1e-5 relative (FP32 sums of squares, as before)."""
+    import torch
+    R = 8192 if row0 > 1000 else 0
+    if R:
+        row0 = R - row0
+    off, ring, fb, rows = _case(ndm, 200, nt, 30.0, 9, 0, row0, R)
+    ave, sig = O.dedisperse_sigma(fb, off, nt)
+    out = torch.full((2, ndm, nt), 7.0, device="cuda")
+    vf.DedispPlan(off)(torch.from_numpy(ring).cuda(), nt, row0=row0, row_mask=R - 1 if R else 0xFFFFFFFF,
+                       nrows_valid=rows, out=out[0], sigma_out=out[1], stats=False)
+    got = out.cpu().numpy()
+    assert np.max(np.abs(got[0] - ave)) <= 1e-5 * np.sqrt(np.mean(ave ** 2))
+    assert np.max(np.abs(got[1] - sig) / sig) <= 1e-5

@@ -376,6 +376,82 @@ int launch_series_stats(const float* dd, int ndm, long long nt, long long stride
   return cuda_status(cudaGetLastError());
 }
 
+// Few trials (and the sigma form of the time-series tool, two trials): nothing to
+// share between trials that the L2 does not share already, so the kernel is made
+// to stream the filterbank.  A CTA owns 32 K samples of one trial; its 16 warps
+// take every 16th channel, lanes run along time and eight channels' loads are in
+// flight per lane, and the warps' sums are added in order at the end.  Trials of
+// the same samples are neighbouring CTAs and walk the channels together, so the
+// second one's reads are L2 hits.  (The staged kernel gives a CTA 16 trials: with
+// two, 7/8 of its warps' slots are idle and 72 CTAs serve 18,211 samples.)
+constexpr int kFewWarps = 16;
+template <typename T, bool SIGMA, int K>
+__global__ void __launch_bounds__(kFewWarps * 32) k_dedisp_few(const DdKParams p) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int d = blockIdx.x;
+  const long long t0 = (long long)blockIdx.y * (32 * K);
+  const int* off = p.off + (long long)d * p.nchan;
+  const T* fb = reinterpret_cast<const T*>(p.fb);
+  const unsigned mask = p.row_mask;
+  unsigned row[K];  // of this lane's samples at delay 0; samples past the end read the last one's rows
+#pragma unroll
+  for (int k = 0; k < K; ++k) row[k] = (unsigned)(p.row0 + min(t0 + lane + 32 * k, p.nt_out - 1));
+  float acc[K], acc2[SIGMA ? K : 1];
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    acc[k] = 0.f;
+    if (SIGMA) acc2[k] = 0.f;
+  }
+  constexpr int U = 8;  // channels in flight
+  for (int c0 = warp; c0 < p.nchan; c0 += kFewWarps * U) {
+    T v[U][K];
+    float w[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int c = min(c0 + kFewWarps * u, p.nchan - 1);
+      const unsigned o = (unsigned)__ldg(off + c);
+      const T* x = fb + (long long)c * p.chan_stride;
+      if (sizeof(T) != 4) w[u] = p.chan_scale ? __ldg(p.chan_scale + c) : p.uniform_scale;
+#pragma unroll
+      for (int k = 0; k < K; ++k) v[u][k] = x[(row[k] + o) & mask];
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      if (c0 + kFewWarps * u < p.nchan) {
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+          const float x = to_f<T>(v[u][k]);
+          if (sizeof(T) == 4) acc[k] += x;
+          else acc[k] = fmaf(w[u], x, acc[k]);
+          if (SIGMA) acc2[k] = fmaf(x, x, acc2[k]);
+        }
+      }
+    }
+  }
+  __shared__ float red[SIGMA ? 2 : 1][kFewWarps][32 * K];
+#pragma unroll
+  for (int k = 0; k < K; ++k) {
+    red[0][warp][lane + 32 * k] = acc[k];
+    if (SIGMA) red[SIGMA ? 1 : 0][warp][lane + 32 * k] = acc2[k];
+  }
+  __syncthreads();
+  const int i = threadIdx.x;
+  const long long t = t0 + i;
+  if (i >= 32 * K || t >= p.nt_out) return;
+  float s = 0.f, q = 0.f;
+#pragma unroll
+  for (int g = 0; g < kFewWarps; ++g) {
+    s += red[0][g][i];
+    if (SIGMA) q += red[SIGMA ? 1 : 0][g][i];
+  }
+  p.out[(long long)d * p.out_stride + t] = s / (float)p.nchan;
+  if (SIGMA) {
+    const double n = (double)p.nchan;
+    const double var = ((double)q - (double)s * (double)s / n) / (n * (n - 1.0));
+    p.sig_out[(long long)d * p.out_stride + t] = (float)sqrt(var > 0.0 ? var : 0.0);
+  }
+}
+
 // Fallback for delay spreads too wide to stage: direct loads, one thread per
 // output sample (lanes along time keep the loads coalesced).
 template <typename T, bool SIGMA>
@@ -486,8 +562,8 @@ struct vfrb_ddplan {
   bool group_ok[5] = {};            // [D]: the groups of D trials apply
   bool groups_built = false;
   int variant[3] = {0, 0, 0};       // chosen variant per storage form (VFRB_DD_*)
-  // AUTO runs the band kernel where it applies (dedisperse_band.cu), else the
-  // fastest of the others when they have been timed, else the default
+  // AUTO runs its own kernels where they apply (launch_auto), else the fastest of
+  // the others when they have been timed, else the default
   int tuned[3] = {0, 0, 0};
   vfrb::BandTables* band = nullptr;
 };
@@ -538,6 +614,33 @@ static int dd_launch_t(const vfrb_ddplan* pl, const vfrb_dd_args& a, DdKParams& 
     k_dedisperse_direct<T, SIGMA><<<grid, 256, 0, s>>>(k);
   }
   return cuda_status(cudaGetLastError());
+}
+
+// Most trials that the streaming kernel takes.  By the trials alone, so that the
+// order of the sums does not change with the number of samples.  Against the band
+// kernel (3908 channels, ms): 16 trials 0.04 / 0.10 / 0.57 against 0.74 / 0.78 /
+// 0.78 at 300 / 2000 / 18,000 samples, 32 trials 0.06 / 0.15 / 1.05 against 0.71 /
+// 0.74 / 0.75.  Sigma form against the staged kernel: 64 trials 0.08 / 0.27 / 2.11
+// against 1.39 / 1.43 / 2.16; two trials x 18,000 (the tool's case) 5.38 -> 0.11.
+constexpr int kFewTrials = 16;
+constexpr int kFewTrialsSigma = 64;
+
+template <typename T, bool SIGMA, int K>
+static int few_launch_k(const vfrb_ddplan* pl, const DdKParams& k, cudaStream_t s, int* launched) {
+  const long long ny = (k.nt_out + 32 * K - 1) / (32 * K);
+  if (ny > 65535) return VFRB_OK;
+  k_dedisp_few<T, SIGMA, K><<<dim3((unsigned)pl->ndm, (unsigned)ny), kFewWarps * 32, 0, s>>>(k);
+  *launched = 1;
+  return cuda_status(cudaGetLastError());
+}
+// samples per lane: four, fewer where the CTAs would not fill the device twice
+// (the order of a sample's sums does not depend on it)
+template <typename T, bool SIGMA>
+static int few_launch_t(const vfrb_ddplan* pl, const DdKParams& k, cudaStream_t s, int* launched) {
+  const long long lanes = k.nt_out * pl->ndm;
+  if (lanes >= 2LL * 148 * 128) return few_launch_k<T, SIGMA, 4>(pl, k, s, launched);
+  if (lanes >= 2LL * 148 * 64) return few_launch_k<T, SIGMA, 2>(pl, k, s, launched);
+  return few_launch_k<T, SIGMA, 1>(pl, k, s, launched);
 }
 
 template <typename T, int D, int TT, int SMAX>
@@ -720,25 +823,7 @@ static int resolve_auto(const vfrb_ddplan* pl, int storage) {
   return pl->tuned[storage] != VFRB_DD_AUTO ? pl->tuned[storage] : default_variant(pl, storage);
 }
 
-// The band kernel for this call, with the statistics from the finished
-// series; *launched = 0 when it does not apply.
-static int launch_band(const vfrb_ddplan* pl, const vfrb_dd_args& a, cudaStream_t s, int* launched) {
-  *launched = 0;
-  if (!pl->band || a.sigma_out) return VFRB_OK;
-  const bool want_stats = a.ave || a.sigma || a.peak || a.frb || a.argmax;
-  const long long ntb = (a.nt_out + kPartNt - 1) / kPartNt;
-  if (want_stats && ntb * pl->ndm > 0x7fffffffLL) return VFRB_OK;
-  const int st = band_launch(pl->band, a, nullptr, 0, s, launched);
-  if (st || !*launched || !want_stats) return st;
-  DmPartial* part = reinterpret_cast<DmPartial*>(a.workspace);
-  k_series_part<<<(unsigned)(ntb * pl->ndm), 256, 0, s>>>(a.out, a.nt_out, a.out_stride, pl->ndm, (int)ntb, part);
-  k_dm_stats<<<(pl->ndm + 7) / 8, 256, 0, s>>>(part, (int)ntb, pl->ndm, a.nt_out, a.ave, a.sigma, a.peak, a.frb,
-                                               a.argmax);
-  return cuda_status(cudaGetLastError());
-}
-
-static int launch_variant(const vfrb_ddplan* pl, int v, const vfrb_dd_args& a, cudaStream_t s,
-                          const void* fb1 = nullptr) {
+static DdKParams dd_params(const vfrb_ddplan* pl, const vfrb_dd_args& a) {
   const bool want_stats = a.ave || a.sigma || a.peak || a.frb || a.argmax;
   DdKParams k{};
   k.fb = a.fb;
@@ -757,6 +842,38 @@ static int launch_variant(const vfrb_ddplan* pl, int v, const vfrb_dd_args& a, c
   k.sig_out = a.sigma_out;
   k.part = want_stats ? reinterpret_cast<DmPartial*>(a.workspace) : nullptr;
   k.err = a.d_err;
+  return k;
+}
+
+// AUTO's own kernels -- streaming for few trials, band-wise for more -- with the
+// statistics from the finished series; *launched = 0 when neither applies.
+static int launch_auto(const vfrb_ddplan* pl, const vfrb_dd_args& a, cudaStream_t s, int* launched) {
+  *launched = 0;
+  const bool want_stats = a.ave || a.sigma || a.peak || a.frb || a.argmax;
+  const long long ntb = (a.nt_out + kPartNt - 1) / kPartNt;
+  if (want_stats && ntb * pl->ndm > 0x7fffffffLL) return VFRB_OK;
+  int st = VFRB_OK;
+  if (pl->ndm <= (a.sigma_out ? kFewTrialsSigma : kFewTrials)) {
+    const DdKParams k = dd_params(pl, a);
+    if (a.sigma_out) st = few_launch_t<float, true>(pl, k, s, launched);
+    else if (a.storage == VFRB_F32) st = few_launch_t<float, false>(pl, k, s, launched);
+    else if (a.storage == VFRB_F16) st = few_launch_t<__half, false>(pl, k, s, launched);
+    else st = few_launch_t<int8_t, false>(pl, k, s, launched);
+  } else if (pl->band && !a.sigma_out) {
+    st = band_launch(pl->band, a, nullptr, 0, s, launched);
+  }
+  if (st || !*launched || !want_stats) return st;
+  DmPartial* part = reinterpret_cast<DmPartial*>(a.workspace);
+  k_series_part<<<(unsigned)(ntb * pl->ndm), 256, 0, s>>>(a.out, a.nt_out, a.out_stride, pl->ndm, (int)ntb, part);
+  k_dm_stats<<<(pl->ndm + 7) / 8, 256, 0, s>>>(part, (int)ntb, pl->ndm, a.nt_out, a.ave, a.sigma, a.peak, a.frb,
+                                               a.argmax);
+  return cuda_status(cudaGetLastError());
+}
+
+static int launch_variant(const vfrb_ddplan* pl, int v, const vfrb_dd_args& a, cudaStream_t s,
+                          const void* fb1 = nullptr) {
+  const bool want_stats = a.ave || a.sigma || a.peak || a.frb || a.argmax;
+  DdKParams k = dd_params(pl, a);
   int ntb = 0, st = VFRB_OK;
   if (!a.sigma_out && (v == VFRB_DD_REG1 || v == VFRB_DD_REG2 || v == VFRB_DD_REG4))
     st = reg_launch(pl, v, a, k.part, s, &ntb);
@@ -800,7 +917,7 @@ int launch_dedisperse_plan(const vfrb_ddplan* pl, const vfrb_dd_args& a, cudaStr
     return VFRB_ERR_ARG;
   if (pl->variant[a.storage] == VFRB_DD_AUTO) {
     int launched = 0;
-    const int st = launch_band(pl, a, s, &launched);
+    const int st = launch_auto(pl, a, s, &launched);
     if (st || launched) return st;
   }
   return launch_variant(pl, resolve_auto(pl, a.storage), a, s, a.fb_shift1);
@@ -819,6 +936,8 @@ int launch_dedisperse_jobs(const vfrb_ddplan* pl, int storage, const DdJob* jobs
   if (!pl || njobs < 1 || njobs > kDdMaxJobs || storage < VFRB_F32 || storage > VFRB_F16) return VFRB_ERR_ARG;
   const int v = resolve_auto(pl, storage);
   const bool band = pl->variant[storage] == VFRB_DD_AUTO && pl->band;
+  // (the streaming kernel has no batched form: the caller launches it per stream)
+  if (pl->variant[storage] == VFRB_DD_AUTO && pl->ndm <= kFewTrials) return VFRB_OK;
   if (!band && v != VFRB_DD_PAT4 && v != VFRB_DD_PAT2) return VFRB_OK;
   vfrb_dd_args a{};
   a.fb = jobs[0].fb;
@@ -913,12 +1032,12 @@ int ddplan_autotune(vfrb_ddplan* pl, int storage, long long nt, float* times, cu
   }
   float best = 1e30f;
   int bestv = VFRB_DD_STAGED;
-  // The band kernel (AUTO) is kept wherever it applies, not timed: it was the
-  // fastest at every size tried (8 to 2048 trials, 300 to 16,384 samples, 1.4 to
-  // 4.6 times the best of the others), and plans made side by side, whose timings
-  // disturb each other, then sum in the same order.
-  int band = 0;
-  if (launch_band(pl, a, s, &band) != VFRB_OK) band = 0;
+  // AUTO's own kernels are kept wherever they apply, not timed: they were the
+  // fastest at every size tried (1 to 2048 trials, 300 to 18,000 samples, 1.4
+  // times the best of the others and more), and plans made side by side, whose
+  // timings disturb each other, then sum in the same order.
+  int own = 0;
+  if (launch_auto(pl, a, s, &own) != VFRB_OK) own = 0;
   if (times) times[VFRB_DD_AUTO] = -1.f;
   // the direct variant last: it is timed only when nothing faster applies
   static const int order[] = {VFRB_DD_STAGED, VFRB_DD_REG1, VFRB_DD_REG2, VFRB_DD_REG4,
@@ -953,7 +1072,7 @@ int ddplan_autotune(vfrb_ddplan* pl, int storage, long long nt, float* times, cu
   cleanup();
   if (err) return err;
   pl->tuned[storage] = bestv;
-  pl->variant[storage] = band ? VFRB_DD_AUTO : bestv;
+  pl->variant[storage] = own ? VFRB_DD_AUTO : bestv;
   return VFRB_OK;
 }
 
