@@ -608,3 +608,40 @@ def test_boxcar_search_matches_oracle(vf, O):
     assert np.allclose(snr.cpu().numpy(), best, rtol=1e-6)
     wp = width[[0, 9, 18, 27, 36]]  # the pulse trials: best width grows with the pulse width
     assert np.all(np.diff(wp) >= 0) and wp[0] == 1 and wp[-1] >= 16
+
+
+def test_subtract_zero_more_channels_than_shared_memory(vf, O):
+    """subtractZERO with more channels than a CTA's shared memory holds rows of,
+    and whole-block subtractbp with more rows: the forms that read memory in
+    every pass, within one float rounding of the FP64 oracle."""
+    torch = _torch()
+    x = _rfi_fb(70, 7200, seed=31)
+    cm = torch.from_numpy(np.ascontiguousarray(x.T)).cuda()
+    vf.subtract_zero(cm)
+    assert np.max(np.abs(cm.cpu().numpy().T - O.subtract_zero(x.astype(np.float64)))) <= 1e-6 * np.abs(x).max()
+    x = _rfi_fb(60000, 12, seed=32)
+    cm = torch.from_numpy(np.ascontiguousarray(x.T)).cuda()
+    vf.subtract_bp_full(cm)
+    ref = O.subtract_bp_full(x.astype(np.float64))
+    got, ok = cm.cpu().numpy().T, ~np.isnan(ref)
+    assert np.array_equal(np.isnan(got), ~ok) and np.max(np.abs(got[ok] - ref[ok])) <= 1e-6 * np.abs(x).max()
+
+
+@pytest.mark.parametrize("rows,ncol,nblk,row0", [(3072, 1024, 3, 0), (2100, 1024, 2, 1500), (5000, 2560, 2, 0),
+                                                 (9000, 6000, 2, 0), (9000, 9000, 1, 3)])
+def test_chan_stats_block_lengths(vf, O, rows, ncol, nblk, row0):
+    """Blocks of exactly 1024 rows, across a ring's end, and of the lengths where
+    the kernel takes more warps per channel or reads the rows in every pass."""
+    torch = _torch()
+    nch = 37
+    x = _rfi_fb(rows, nch, seed=rows)
+    x[rows // 2, 3] = 1e4
+    R = 16384
+    ring = torch.zeros((nch, R), device="cuda")
+    r0 = R - row0 if row0 else 0
+    ring[:, torch.from_numpy((r0 + np.arange(rows)) % R).cuda()] = torch.from_numpy(np.ascontiguousarray(x.T)).cuda()
+    a, s, o = vf.chan_stats(ring, rows, ncol, nblk, row0=r0, row_mask=R - 1)
+    a_r, s_r, o_r = O.calcstats_chan(x.astype(np.float64), ncol, nblk)
+    assert np.max(np.abs(a.cpu().numpy() - a_r)) <= 1e-6 * np.abs(x).max()
+    assert np.max(np.abs(s.cpu().numpy() - s_r) / np.maximum(s_r, 1e-12)) <= 1e-6 or np.allclose(s.cpu(), s_r, rtol=1e-6, atol=1e-9)
+    assert np.array_equal(o.cpu().numpy(), o_r)
