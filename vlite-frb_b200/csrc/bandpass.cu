@@ -3,18 +3,26 @@
 //
 // K2 replaces subtractbpCAL (PIPE:1427-1474; STATS:869-908; TS:1365-1407).
 // A CTA takes one window of <=128 rows x 32 channels of the raw time-major
-// filterbank (coalesced 128-byte row segments), transposes it in shared
-// memory, and one warp per channel computes in FP64: mean, the variance the
-// reference calls "sig", the open-interval clip ave +- 3 sig and the clipped
-// mean (count floored at 1).  The subtracted rows are written channel-major
-// (512-byte runs per channel), the layout the dedisperser streams, in FP32,
-// FP16 (z = x/s_c) or int8 (round(z*q)) form.  subtract_mode 1 skips the
-// statistics and writes the rows unchanged (the input of the whole-block
-// subtractbp in rfi.cu).  The FP16 form can also write a copy shifted by one
-// row, out1[c][r - 1] = out[c][r] (absolute rows, the same ring geometry):
-// with both copies the dedisperser reads any window of halves with aligned
-// 4-byte loads.
+// filterbank (coalesced 128-byte row segments), transposes it in shared memory,
+// and computes in FP64: mean, the variance the reference calls "sig", the
+// open-interval clip ave +- 3 sig and the clipped mean (count floored at 1).  Eight
+// lanes share a channel, 16 rows each, so a sum takes three shuffles and four
+// channels reduce at once, and a row is converted to FP64 once.  (A warp per
+// channel, four rows per lane, spent more on its five-step reductions than on the
+// rows.)  The subtracted rows are written channel-major (512-byte runs per
+// channel), the layout the dedisperser streams, in FP32, FP16 (z = x/s_c) or int8
+// (round(z*q)) form.  subtract_mode 1 skips the statistics and writes the rows
+// unchanged (the input of the whole-block subtractbp in rfi.cu).  The FP16 form
+// can also write a copy shifted by one row, out1[c][r - 1] = out[c][r] (absolute
+// rows, the same ring geometry): with both copies the four-trial pattern kernel
+// reads any window of halves with aligned 4-byte loads.
+//
+// Bound by instruction issue: it was 50 instructions per value, most of them row
+// addresses through the rings' masks; where a window does not wrap a ring (all but
+// one in a ring's length) rows are pointer steps.
 #include "vfrb_common.cuh"
+
+#include <algorithm>
 
 namespace vfrb {
 
@@ -27,126 +35,203 @@ __device__ __forceinline__ double warp_sum(double v) {
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
 }
-__device__ __forceinline__ int warp_sum_i(int v) {
+// over each eight neighbouring lanes
+__device__ __forceinline__ double sum8(double v) {
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  for (int o = 4; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
 }
 
 template <int STORAGE>
-__global__ void __launch_bounds__(kBpThreads) k_bandpass(const vfrb_bp_args a, __half* __restrict__ out1) {
-  __shared__ float tile[kBpChan][kBpMaxWin + 1];
+struct BpOut;
+template <>
+struct BpOut<VFRB_F32> {
+  using T = float;
+  __device__ static T of(float y, float, float) { return y; }
+};
+template <>
+struct BpOut<VFRB_F16> {
+  using T = __half;
+  __device__ static T of(float y, float inv, float) { return __float2half_rn(y * inv); }
+};
+template <>
+struct BpOut<VFRB_I8> {
+  using T = int8_t;
+  __device__ static T of(float y, float inv, float q) {
+    return (int8_t)fminf(fmaxf(rintf(y * inv * q), -127.f), 127.f);
+  }
+};
+
+// FULL: the window has kBpMaxWin rows and every channel of the tile exists
+template <int STORAGE, bool FULL>
+__device__ __forceinline__ void bp_window(const vfrb_bp_args& a, __half* __restrict__ out1,
+                                          float (&tile)[kBpChan][kBpMaxWin + 1]) {
+  using T = typename BpOut<STORAGE>::T;
+  constexpr int kWarps = kBpThreads / 32;
+  constexpr int kRows = kBpMaxWin / kWarps;  // rows a warp loads, and rows a lane sums
   const int win = blockIdx.y;
   const int c0 = blockIdx.x * kBpChan;
   const long long r0 = (long long)win * a.window;
-  const int npts = (int)min((long long)a.window, (long long)a.nrows - r0);
+  const int npts = FULL ? kBpMaxWin : (int)min((long long)a.window, (long long)a.nrows - r0);
+  const int nc = FULL ? kBpChan : min(kBpChan, a.nchan - c0);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  int err = 0;
 
-  // load rows (time-major) -> tile[ch][row]: a warp's 16 rows are loaded
-  // into registers first, so all 16 row segments are in flight together
+  // rows (time-major) -> tile[ch][row]: a warp's 16 rows are loaded into registers
+  // first, so all 16 row segments are in flight together
   {
-    constexpr int kRowsPerWarp = kBpMaxWin / (kBpThreads / 32);
-    float v[kRowsPerWarp];
-    const int c = c0 + lane;
+    float v[kRows];
+    const unsigned long long first = (unsigned long long)(a.in_row0 + r0) & (unsigned long long)a.in_row_mask;
+    if (FULL && first + kBpMaxWin <= (unsigned long long)a.in_row_mask + 1ULL) {
+      const float* src = a.in + (long long)(first + warp) * a.in_row_stride + c0 + lane;
+      const long long step = kWarps * a.in_row_stride;
 #pragma unroll
-    for (int k = 0; k < kRowsPerWarp; ++k) {
-      const int r = warp + (kBpThreads / 32) * k;
-      const unsigned long long rr = (unsigned long long)(a.in_row0 + r0 + r) & (unsigned long long)a.in_row_mask;
-      v[k] = (r < npts && c < a.nchan) ? a.in[(long long)rr * a.in_row_stride + c] : 0.f;
+      for (int k = 0; k < kRows; ++k) {
+        v[k] = *src;
+        src += step;
+      }
+    } else {
+#pragma unroll
+      for (int k = 0; k < kRows; ++k) {
+        const int r = warp + kWarps * k;
+        const unsigned long long rr = (unsigned long long)(a.in_row0 + r0 + r) & (unsigned long long)a.in_row_mask;
+        v[k] = (r < npts && lane < nc) ? a.in[(long long)rr * a.in_row_stride + c0 + lane] : 0.f;
+      }
     }
 #pragma unroll
-    for (int k = 0; k < kRowsPerWarp; ++k) {
-      const int r = warp + (kBpThreads / 32) * k;
-      if (r < npts) tile[lane][r] = v[k];
-    }
+    for (int k = 0; k < kRows; ++k) tile[lane][warp + kWarps * k] = v[k];
   }
   __syncthreads();
 
-  for (int cl = warp; cl < kBpChan; cl += kBpThreads / 32) {
-    const int c = c0 + cl;
-    if (c >= a.nchan) break;
-    float x[kBpMaxWin / 32];
-    double s = 0.0;
-#pragma unroll
-    for (int k = 0; k < kBpMaxWin / 32; ++k) {
-      const int r = lane + 32 * k;
-      x[k] = (r < npts) ? tile[cl][r] : 0.f;
-      s += (r < npts) ? (double)x[k] : 0.0;
-    }
+  if (a.subtract_mode == 0 || a.win_mean || a.win_var) {
+    // lanes g, g + 8, ... of channel cl = warp + 8 (lane / 8): with the tile's odd
+    // pitch the 32 lanes of a load touch 32 banks
+    const int g = lane & 7, cl = warp + kWarps * (lane >> 3);
+    float* row = tile[cl] + g;
     double cave = 0.0, sig = 0.0;  // subtract_mode 1: copy only (cave = 0)
     if (a.subtract_mode == 0) {
+      float x[kRows];
+      double xd[kRows];
+      double s = 0.0;
+#pragma unroll
+      for (int k = 0; k < kRows; ++k) {
+        x[k] = row[8 * k];  // rows past the window hold zeros
+        xd[k] = (double)x[k];
+        s += xd[k];
+      }
       const double n = (double)npts;
-      const double ave = warp_sum(s) / n;
+      s = sum8(s);
+      const double ave = s / n;
       double sd = 0.0, sd2 = 0.0;
 #pragma unroll
-      for (int k = 0; k < kBpMaxWin / 32; ++k) {
-        const int r = lane + 32 * k;
-        if (r < npts) {
-          const double d = (double)x[k] - ave;
+      for (int k = 0; k < kRows; ++k) {
+        if (FULL || g + 8 * k < npts) {
+          const double d = xd[k] - ave;
           sd += d;
           sd2 += d * d;
         }
       }
-      sd = warp_sum(sd);
-      sd2 = warp_sum(sd2);
+      sd = sum8(sd);
+      sd2 = sum8(sd2);
       sig = (sd2 - (sd * sd) / n) / (n - 1.0);  // variance, NaN when npts == 1
-      const double hi = ave + 3.0 * sig, lo = ave - 3.0 * sig;
-      double cs = 0.0;
-      int cnt = 0;
+      // the clip decided in FP32: the thresholds rounded outwards order every float alike
+      const float hi = __double2float_ru(ave + 3.0 * sig), lo = __double2float_rd(ave - 3.0 * sig);
+      bool all = true;
+#pragma unroll
+      for (int k = 0; k < kRows; ++k)
+        if (FULL || g + 8 * k < npts) all = all && x[k] < hi && x[k] > lo;
+      double cnt = n, cs = s;
+      if (!__all_sync(0xffffffffu, all)) {  // some channel of the warp loses rows
+        int kept = 0;
+        cs = 0.0;
+#pragma unroll
+        for (int k = 0; k < kRows; ++k)
+          if ((FULL || g + 8 * k < npts) && x[k] < hi && x[k] > lo) {
+            cs += xd[k];
+            ++kept;
+          }
+        cs = sum8(cs);
+        cnt = sum8((double)kept);
+        if (cnt == 0.0) cnt = 1.0;
+      }
+      cave = cs / cnt;
+#pragma unroll
+      for (int k = 0; k < kRows; ++k) row[8 * k] = (float)(xd[k] - cave);
+    }
+    if (g == 0 && cl < nc) {
+      if (a.win_mean) a.win_mean[(long long)win * a.nchan + c0 + cl] = (float)cave;
+      if (a.win_var) a.win_var[(long long)win * a.nchan + c0 + cl] = (float)sig;
+    }
+    __syncthreads();
+  }
+
+  // tile -> channel-major rows, a warp per channel
+  const unsigned long long omask = (unsigned long long)a.out_row_mask;
+  const unsigned long long first = (unsigned long long)(a.out_row0 + r0) & omask;
+  const bool straight = FULL && first + kBpMaxWin <= omask + 1ULL;
+  T* const out = reinterpret_cast<T*>(a.out);
+#pragma unroll 1
+  for (int cl = warp; cl < nc; cl += kWarps) {
+    const float inv = (STORAGE == VFRB_F32) ? 1.f : a.inv_scale[c0 + cl];
+    T* dst = out + (long long)(c0 + cl) * a.out_chan_stride;
+    const float* row = tile[cl];
+    if (straight && STORAGE == VFRB_F16 && ((uintptr_t)(dst + first) & 3) == 0) {
+      // two rows per store; the shifted copy's pairs (rows 2i + 1, 2i + 2) start where
+      // this one's do, and its row before the window and the window's last row alone
+      __half2* d2 = reinterpret_cast<__half2*>(dst + first);
+      __half* d1 = out1 ? out1 + (long long)(c0 + cl) * a.out_chan_stride : nullptr;
+#pragma unroll
+      for (int k = 0; k < kBpMaxWin / 64; ++k) {
+        const int i = lane + 32 * k;
+        const __half lo = __float2half_rn(row[2 * i] * inv), hi = __float2half_rn(row[2 * i + 1] * inv);
+        d2[i] = __halves2half2(lo, hi);
+        if (d1) {
+          const __half up = __shfl_down_sync(0xffffffffu, lo, 1);  // row 2i + 2 of the next lane
+          if (lane < 31) {
+            if (((uintptr_t)(d1 + first) & 3) == 0) {
+              reinterpret_cast<__half2*>(d1 + first)[i] = __halves2half2(hi, up);
+            } else {
+              d1[first + 2 * i] = hi;
+              d1[first + 2 * i + 1] = up;
+            }
+          } else {
+            d1[first + 2 * i] = hi;
+            if (2 * i + 2 < kBpMaxWin) d1[first + 2 * i + 1] = __float2half_rn(row[2 * i + 2] * inv);
+          }
+          if (i == 0 && a.out_row0 + r0 >= 1)
+            d1[(unsigned long long)(a.out_row0 + r0 - 1) & omask] = lo;
+        }
+      }
+    } else {
 #pragma unroll
       for (int k = 0; k < kBpMaxWin / 32; ++k) {
         const int r = lane + 32 * k;
-        const double xv = (double)x[k];
-        if (r < npts && xv < hi && xv > lo) {
-          cs += xv;
-          ++cnt;
-        }
-      }
-      cs = warp_sum(cs);
-      cnt = warp_sum_i(cnt);
-      if (cnt == 0) cnt = 1;
-      cave = cs / (double)cnt;
-    }
-    if (lane == 0) {
-      if (a.win_mean) a.win_mean[(long long)win * a.nchan + c] = (float)cave;
-      if (a.win_var) a.win_var[(long long)win * a.nchan + c] = (float)sig;
-    }
-    const float inv = (STORAGE == VFRB_F32) ? 1.f : a.inv_scale[c];
-#pragma unroll
-    for (int k = 0; k < kBpMaxWin / 32; ++k) {
-      const int r = lane + 32 * k;
-      if (r < npts) {
-        const float y = (float)((double)x[k] - cave);
-        const unsigned long long orow =
-            (unsigned long long)(a.out_row0 + r0 + r) & (unsigned long long)a.out_row_mask;
-        const long long o = (long long)c * a.out_chan_stride + (long long)orow;
-        if (STORAGE == VFRB_F32) {
-          reinterpret_cast<float*>(a.out)[o] = y;
-        } else if (STORAGE == VFRB_F16) {
-          const __half h = __float2half_rn(y * inv);
-          reinterpret_cast<__half*>(a.out)[o] = h;
+        if (FULL || r < npts) {
+          const T v = BpOut<STORAGE>::of(row[r], inv, a.q_scale);
           const long long ra = a.out_row0 + r0 + r;  // absolute row; row ra - 1 of the shifted copy
-          if (out1 && ra >= 1)
-            out1[(long long)c * a.out_chan_stride +
-                 (long long)((unsigned long long)(ra - 1) & (unsigned long long)a.out_row_mask)] = h;
-        } else {
-          float q = rintf(y * inv * a.q_scale);
-          q = fminf(fmaxf(q, -127.f), 127.f);
-          reinterpret_cast<int8_t*>(a.out)[o] = (int8_t)q;
+          if (straight) dst[first + r] = v;
+          else dst[(unsigned long long)ra & omask] = v;
+          if constexpr (STORAGE == VFRB_F16) {
+            if (out1 && ra >= 1)
+              out1[(long long)(c0 + cl) * a.out_chan_stride + (long long)((unsigned long long)(ra - 1) & omask)] = v;
+          }
         }
-        if (a.tm_out) tile[cl][r] = y;
       }
     }
   }
   if (a.tm_out) {
-    __syncthreads();
-    for (int r = warp; r < npts; r += kBpThreads / 32) {
-      const int c = c0 + lane;
-      if (c < a.nchan) a.tm_out[(r0 + r) * a.tm_row_stride + c] = tile[lane][r];
-    }
+    for (int r = warp; r < npts; r += kWarps)
+      if (lane < nc) a.tm_out[(r0 + r) * a.tm_row_stride + c0 + lane] = tile[lane][r];
   }
-  if (err && a.d_err) atomicOr(a.d_err, err);
+}
+
+template <int STORAGE>
+__global__ void __launch_bounds__(kBpThreads) k_bandpass(const __grid_constant__ vfrb_bp_args a,
+                                                         __half* __restrict__ out1) {
+  __shared__ float tile[kBpChan][kBpMaxWin + 1];
+  const bool full = a.window == kBpMaxWin && (long long)(blockIdx.y + 1) * kBpMaxWin <= a.nrows &&
+                    ((int)blockIdx.x + 1) * kBpChan <= a.nchan;
+  if (full) bp_window<STORAGE, true>(a, out1, tile);
+  else bp_window<STORAGE, false>(a, out1, tile);
 }
 
 int launch_bandpass(const vfrb_bp_args& a, cudaStream_t s) {
@@ -167,46 +252,94 @@ int launch_bandpass(const vfrb_bp_args& a, cudaStream_t s) {
 }
 
 // ---- K4: per-channel statistics (STATS:910-946) ---------------------------
-// One warp per (channel, statistics block); the block's rows are contiguous
-// in the channel-major layout.  FP64 mean and variance; the outlier count
-// uses the reference's float comparison x > ave + 5*sig and stores the
-// integer quotient count/npts.
-__global__ void __launch_bounds__(256) k_chan_stats(const vfrb_cs_args a) {
-  const int lane = threadIdx.x & 31;
-  const long long gw = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
-  if (gw >= (long long)a.nchan * a.nstatblks) return;
-  const int c = (int)(gw % a.nchan);
-  const int k = (int)(gw / a.nchan);
+// NW warps per (channel, statistics block); the block's rows are contiguous in
+// the channel-major layout.  FP64 mean and variance; the outlier count uses the
+// reference's float comparison x > ave + 5*sig (decided in FP32 against the
+// threshold rounded down, which orders every float alike) and stores the integer
+// quotient count/npts.  The rows are kept in registers (32 per lane, all loads in
+// flight at once) over the three passes; blocks too long for that (NW = 0: one
+// warp) read them three times.  FULL: every block has exactly the registers' rows.
+template <int NW, bool FULL>
+__global__ void __launch_bounds__(256) k_chan_stats(const __grid_constant__ vfrb_cs_args a) {
+  constexpr int G = NW ? NW : 1;  // warps per (channel, block)
+  constexpr int R = 32;
+  __shared__ double red[2][8];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int gl = (int)(threadIdx.x % (32 * G));  // thread of the group
+  const long long gw = (long long)blockIdx.x * (8 / G) + warp / G;
+  const bool live = gw < (long long)a.nchan * a.nstatblks;
+  const int c = live ? (int)(gw % a.nchan) : 0;
+  const int k = live ? (int)(gw / a.nchan) : 0;
   const long long colmin = (long long)a.ncolstatblk * k;
   long long colmax = colmin + a.ncolstatblk;
   if (colmax > a.nrows) colmax = a.nrows;
   const int npts = (int)(colmax - colmin);
   const float* base = a.fb + (long long)c * a.chan_stride;
-  auto at = [&](long long r) {
-    return base[(unsigned long long)(a.row0 + r) & (unsigned long long)a.row_mask];
+  const unsigned r0 = (unsigned)(a.row0 + colmin);  // ring rows are 32-bit
+  auto at = [&](int i) { return base[(r0 + (unsigned)i) & a.row_mask]; };
+  // sums over the group's warps, the same on every lane
+  auto group_sum = [&](double& u, double& v) {
+    u = warp_sum(u);
+    v = warp_sum(v);
+    if (G == 1) return;
+    __syncthreads();
+    if (lane == 0) {
+      red[0][warp] = u;
+      red[1][warp] = v;
+    }
+    __syncthreads();
+    u = v = 0.0;
+#pragma unroll
+    for (int w = 0; w < G; ++w) {
+      u += red[0][warp / G * G + w];
+      v += red[1][warp / G * G + w];
+    }
   };
-  double s = 0.0;
-  for (long long r = colmin + lane; r < colmax; r += 32) s += (double)at(r);
+  float x[NW ? R : 1];
+  auto each = [&](auto&& f) {
+    if constexpr (NW != 0) {
+#pragma unroll
+      for (int i = 0; i < R; ++i)
+        if (FULL || gl + 32 * G * i < npts) f(x[i]);
+    } else {
+      for (int i = gl; i < npts; i += 32) f(at(i));
+    }
+  };
+  if constexpr (NW != 0) {
+    const unsigned long long first = r0 & a.row_mask;
+    if (FULL && first + 32 * G * R <= (unsigned long long)a.row_mask + 1ULL) {  // the rows do not wrap the ring
+      const float* src = base + first + gl;
+#pragma unroll
+      for (int i = 0; i < R; ++i) x[i] = src[32 * G * i];
+    } else {
+#pragma unroll
+      for (int i = 0; i < R; ++i) x[i] = FULL || gl + 32 * G * i < npts ? at(gl + 32 * G * i) : 0.f;
+    }
+  }
+  double s = 0.0, none = 0.0;
+  each([&](float v) { s += (double)v; });
+  group_sum(s, none);
   const double n = (double)npts;
-  const double ave = warp_sum(s) / n;
+  const double ave = s / n;
   double sd = 0.0, sd2 = 0.0;
-  for (long long r = colmin + lane; r < colmax; r += 32) {
-    const double d = (double)at(r) - ave;
+  each([&](float v) {
+    const double d = (double)v - ave;
     sd += d;
     sd2 += d * d;
-  }
-  sd = warp_sum(sd);
-  sd2 = warp_sum(sd2);
+  });
+  group_sum(sd, sd2);
   const double sig = (sd2 - sd * sd / n) / (n - 1.0);
-  const double hi = ave + 5.0 * sig;
-  int cnt = 0;
-  for (long long r = colmin + lane; r < colmax; r += 32) cnt += ((double)at(r) > hi) ? 1 : 0;
-  cnt = warp_sum_i(cnt);
-  if (lane == 0) {
+  const float hi = __double2float_rd(ave + 5.0 * sig);  // x > hi of a float: x > the threshold rounded down
+  int out = 0;
+  each([&](float v) { out += v > hi ? 1 : 0; });
+  double cnt = (double)out;
+  none = 0.0;
+  group_sum(cnt, none);
+  if (live && gl == 0) {
     const long long o = (long long)k * a.nchan + c;
     a.ave[o] = (float)ave;
     a.sig[o] = (float)sig;
-    a.outlier[o] = (float)(npts > 0 ? cnt / npts : 0);
+    a.outlier[o] = (float)(npts > 0 ? (int)cnt / npts : 0);
   }
 }
 
@@ -215,7 +348,13 @@ int launch_chan_stats(const vfrb_cs_args& a, cudaStream_t s) {
     return VFRB_ERR_ARG;
   if ((long long)a.ncolstatblk * (a.nstatblks - 1) >= a.nrows) return VFRB_ERR_ARG;
   const long long nw = (long long)a.nchan * a.nstatblks;
-  k_chan_stats<<<(unsigned)((nw + 7) / 8), 256, 0, s>>>(a);
+  const int rows = std::min(a.ncolstatblk, a.nrows);  // of the longest block
+  if (rows == 1024 && (long long)rows * a.nstatblks <= a.nrows)
+    k_chan_stats<1, true><<<(unsigned)((nw + 7) / 8), 256, 0, s>>>(a);
+  else if (rows <= 1024) k_chan_stats<1, false><<<(unsigned)((nw + 7) / 8), 256, 0, s>>>(a);
+  else if (rows <= 4096) k_chan_stats<4, false><<<(unsigned)((nw + 1) / 2), 256, 0, s>>>(a);
+  else if (rows <= 8192) k_chan_stats<8, false><<<(unsigned)nw, 256, 0, s>>>(a);
+  else k_chan_stats<0, false><<<(unsigned)((nw + 7) / 8), 256, 0, s>>>(a);
   return cuda_status(cudaGetLastError());
 }
 
@@ -227,21 +366,51 @@ int launch_chan_stats(const vfrb_cs_args& a, cudaStream_t s) {
 //   SK = (M*nsum + 1)/(M - 1) * (M*S2/S1^2 - 1),
 // whose expectation is 1 for Gaussian noise; narrowband RFI drives it below 1
 // (steady tones) or far above it (bursts); a one-row block gives inf/NaN as
-// M - 1 = 0.  FP64 sums.  The FB is time-major,
-// so a warp reads 32 consecutive channels of a row: 128-byte segments.
-__global__ void __launch_bounds__(256) k_chan_sk(const float* __restrict__ fb, long long row_stride, long long row0,
-                                                 unsigned long long row_mask, int nchan, int nrows, int ncolstatblk,
-                                                 int nstatblks, double nsum, float* __restrict__ sk) {
-  const int c = blockIdx.x * 256 + threadIdx.x;
+// M - 1 = 0.  FP64 sums.  The FB is time-major, so a warp reads 32 consecutive
+// channels of a row: 128-byte segments.
+// A CTA takes 64 channels of one block: 16 sets of threads share its rows out
+// (set g rows g, g + 16, ..., eight loads in flight per thread), and the sets'
+// sums are added in order.  (A thread per channel alone gives 175 CTAs of 1024
+// serial loads at 6250 channels x 7 blocks.)
+constexpr int kSkChan = 64, kSkSets = 16;
+__global__ void __launch_bounds__(kSkChan * kSkSets) k_chan_sk(const float* __restrict__ fb, long long row_stride,
+                                                               long long row0, unsigned long long row_mask, int nchan,
+                                                               int nrows, int ncolstatblk, int nstatblks, double nsum,
+                                                               float* __restrict__ sk) {
+  __shared__ double red[2][kSkSets][kSkChan];
+  const int cl = threadIdx.x % kSkChan, g = threadIdx.x / kSkChan;
+  const int c = blockIdx.x * kSkChan + cl;
   const int k = blockIdx.y;
-  if (c >= nchan || k >= nstatblks) return;
   const long long r0 = (long long)ncolstatblk * k;
   const long long r1 = min(r0 + ncolstatblk, (long long)nrows);
+  const float* x = fb + min(c, nchan - 1);
+  auto at = [&](long long r) { return x[(long long)((unsigned long long)(row0 + r) & row_mask) * row_stride]; };
   double s1 = 0.0, s2 = 0.0;
-  for (long long r = r0; r < r1; ++r) {
-    const double x = (double)fb[(long long)((unsigned long long)(row0 + r) & row_mask) * row_stride + c];
-    s1 += x;
-    s2 += x * x;
+  long long r = r0 + g;
+  constexpr int U = 8;
+  for (; r + (U - 1) * kSkSets < r1; r += U * kSkSets) {
+    float v[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) v[u] = at(r + u * kSkSets);
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const double d = (double)v[u];
+      s1 += d;
+      s2 += d * d;
+    }
+  }
+  for (; r < r1; r += kSkSets) {
+    const double d = (double)at(r);
+    s1 += d;
+    s2 += d * d;
+  }
+  red[0][g][cl] = s1;
+  red[1][g][cl] = s2;
+  __syncthreads();
+  if (g != 0 || c >= nchan) return;
+  for (int q = 1; q < kSkSets; ++q) {
+    s1 += red[0][q][cl];
+    s2 += red[1][q][cl];
   }
   const double m = (double)(r1 - r0);
   const double v = (m * nsum + 1.0) / (m - 1.0) * (m * s2 / (s1 * s1) - 1.0);
@@ -255,8 +424,8 @@ int launch_chan_sk_ring(const float* fb_tm, long long row_stride, long long row0
   if (!fb_tm || !sk || nchan <= 0 || nstatblks <= 0 || ncolstatblk <= 1 || nsum < 1 || row_stride < nchan ||
       (long long)nrows - (long long)ncolstatblk * (nstatblks - 1) < 1 || nstatblks > 65535 || row0 < 0)
     return VFRB_ERR_ARG;
-  dim3 grid((unsigned)((nchan + 255) / 256), (unsigned)nstatblks);
-  k_chan_sk<<<grid, 256, 0, s>>>(fb_tm, row_stride, row0, row_mask, nchan, nrows, ncolstatblk, nstatblks,
+  dim3 grid((unsigned)((nchan + kSkChan - 1) / kSkChan), (unsigned)nstatblks);
+  k_chan_sk<<<grid, kSkChan * kSkSets, 0, s>>>(fb_tm, row_stride, row0, row_mask, nchan, nrows, ncolstatblk, nstatblks,
                                  (double)nsum, sk);
   return cuda_status(cudaGetLastError());
 }
@@ -267,31 +436,45 @@ int launch_chan_sk(const float* fb_tm, long long row_stride, int nchan, int nrow
 }
 
 // ---- channel-major -> time-major copy ---------------------------------------
+// Tiles of 64 x 64: each warp has eight 256-byte runs' loads in flight before it
+// stores the first to the tile (a 32 x 32 tile with four loads per thread ran at
+// 45% of the copy rate).
 __global__ void __launch_bounds__(256) k_transpose(const float* __restrict__ src, long long chan_stride,
                                                    unsigned row_mask, long long row0, int nchan, int nrows,
                                                    float* __restrict__ dst, long long dst_row_stride) {
-  __shared__ float t[32][33];
-  const int cb = blockIdx.x * 32, rb = blockIdx.y * 32;
-  const int lx = threadIdx.x & 31, ly = threadIdx.x >> 5;
-  for (int i = ly; i < 32; i += 8) {
-    const int c = cb + i, r = rb + lx;
-    t[i][lx] = (c < nchan && r < nrows)
-                   ? src[(long long)c * chan_stride +
-                         (long long)((unsigned long long)(row0 + r) & (unsigned long long)row_mask)]
-                   : 0.f;
-  }
+  constexpr int T = 64;
+  __shared__ float t[T][T + 1];
+  const int cb = blockIdx.x * T, rb = blockIdx.y * T;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const unsigned r = (unsigned)(row0 + rb + lane);
+  float v[T / 8][2];
+#pragma unroll
+  for (int i = 0; i < T / 8; ++i)
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int c = cb + warp + 8 * i;
+      v[i][h] = (c < nchan && rb + lane + 32 * h < nrows) ? src[(long long)c * chan_stride + ((r + 32u * h) & row_mask)]
+                                                          : 0.f;
+    }
+#pragma unroll
+  for (int i = 0; i < T / 8; ++i)
+#pragma unroll
+    for (int h = 0; h < 2; ++h) t[warp + 8 * i][lane + 32 * h] = v[i][h];
   __syncthreads();
-  for (int i = ly; i < 32; i += 8) {
-    const int r = rb + i, c = cb + lx;
-    if (c < nchan && r < nrows) dst[(long long)r * dst_row_stride + c] = t[lx][i];
-  }
+#pragma unroll
+  for (int i = 0; i < T / 8; ++i)
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int row = rb + warp + 8 * i, c = cb + lane + 32 * h;
+      if (row < nrows && c < nchan) dst[(long long)row * dst_row_stride + c] = t[lane + 32 * h][warp + 8 * i];
+    }
 }
 
 int launch_fb_transpose(const float* src_cm, long long chan_stride, unsigned row_mask, long long row0, int nchan,
                         int nrows, float* dst_tm, long long dst_row_stride, cudaStream_t s) {
   if (!src_cm || !dst_tm || nchan <= 0 || nrows < 0) return VFRB_ERR_ARG;
   if (nrows == 0) return VFRB_OK;
-  dim3 grid((nchan + 31) / 32, (nrows + 31) / 32);
+  dim3 grid((nchan + 63) / 64, (nrows + 63) / 64);
   k_transpose<<<grid, 256, 0, s>>>(src_cm, chan_stride, row_mask, row0, nchan, nrows, dst_tm, dst_row_stride);
   return cuda_status(cudaGetLastError());
 }
