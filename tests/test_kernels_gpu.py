@@ -645,3 +645,53 @@ def test_chan_stats_block_lengths(vf, O, rows, ncol, nblk, row0):
     assert np.max(np.abs(a.cpu().numpy() - a_r)) <= 1e-6 * np.abs(x).max()
     assert np.max(np.abs(s.cpu().numpy() - s_r) / np.maximum(s_r, 1e-12)) <= 1e-6 or np.allclose(s.cpu(), s_r, rtol=1e-6, atol=1e-9)
     assert np.array_equal(o.cpu().numpy(), o_r)
+
+
+@pytest.mark.parametrize("nave", [2, 3, 4, 8, 10])
+def test_channelise_few_rows_equal_many(vf, nave):
+    """A call of few rows (a cluster of NAVE CTAs per row) gives the rows of a
+    larger call (a CTA per row) bit for bit, at the row counts around the change."""
+    torch = _torch()
+    rows = 200
+    L = vf.layout(nave=nave, muoslowfreq=384.0)
+    npairs = (rows * nave * 12500 + 4999) // 5000
+    g = torch.Generator(device="cuda").manual_seed(nave)
+    fr = torch.randint(0, 256, (npairs * 2 * 5032,), dtype=torch.uint8, device="cuda", generator=g)
+    s0 = torch.arange(npairs, dtype=torch.int64, device="cuda") * 10064 + 32
+    many = vf.channelise(fr, s0, s0 + 5032, 0, rows, L)
+    edge = 148 * 7 // 8 // nave
+    for n in {1, edge, edge + 1}:
+        few = vf.channelise(fr, s0, s0 + 5032, 0, n, L)
+        assert torch.equal(few, many[:n]), n
+    few = vf.channelise(fr, s0, s0 + 5032, 5 * nave * 12500, 3, L)
+    assert torch.equal(few, many[5:8])
+
+
+def test_channelise_payload_alignments(vf):
+    """Payloads at offsets 0 and 4 mod 8 (8- and 4-byte staging copies), per pol and
+    mixed, with fill frames among them: the same rows bit for bit."""
+    torch = _torch()
+    rows, nave = 6, 3
+    L = vf.layout(nave=nave, muoslowfreq=384.0)
+    ns = (rows * nave * 12500 + 8 + 4999) // 5000
+    g = torch.Generator(device="cuda").manual_seed(3)
+    pay = torch.randint(0, 256, (2, ns, 5000), dtype=torch.uint8, device="cuda", generator=g)
+    want = {}
+    for name, gap in (("eight", 0), ("four", 4), ("mixed", None)):
+        step = 5032 + (gap or 0)
+        pos = torch.arange(2 * ns, dtype=torch.int64) * step + 32
+        if gap is None:
+            pos += (torch.arange(2 * ns) % 3 == 0) * 4
+        buf = torch.zeros(2 * ns * 5040 + 64, dtype=torch.uint8, device="cuda")
+        for p in range(2):
+            for k in range(ns):
+                a = int(pos[2 * k + p])
+                buf[a:a + 5000] = pay[p, k]
+        s = pos.cuda()
+        s0, s1 = s[0::2].contiguous(), s[1::2].contiguous()
+        s1[4] = -1
+        for sample0 in (0, 4, 8):
+            err = torch.zeros(1, dtype=torch.int32, device="cuda")
+            got = vf.channelise(buf, s0, s1, sample0, rows, L, d_err=err)
+            assert int(err.item()) == 0
+            assert torch.equal(want.setdefault(sample0, got), got), (name, sample0)

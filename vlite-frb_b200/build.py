@@ -65,7 +65,7 @@ def _run(cmd):
 
 def gen_codelets():
     gen = os.path.join(CSRC, "gen_dft.py")
-    out = os.path.join(CSRC, "dft_pairs.cuh")
+    out = os.path.join(CSRC, "dft_codelets.cuh")
     if _newer(gen, out):
         txt = subprocess.run([sys.executable, gen], capture_output=True, text=True, check=True).stdout
         with open(out, "w") as f:

@@ -1,0 +1,110 @@
+// Generated by gen_dft.py -- do not edit by hand.
+// Forward DFT codelets (W = exp(-2*pi*i/N)) in registers.
+#pragma once
+#include <cuda_runtime.h>
+
+namespace vfrb {
+
+struct Cx {
+  float re, im;
+};
+
+// v *= c + i*s
+__device__ __forceinline__ void cx_mul(Cx& v, float c, float s) {
+  const float re = fmaf(-v.im, s, v.re * c);
+  v.im = fmaf(v.re, s, v.im * c);
+  v.re = re;
+}
+__device__ __forceinline__ Cx cx_prod(Cx a, Cx b) {
+  return Cx{fmaf(-a.im, b.im, a.re * b.re), fmaf(a.re, b.im, a.im * b.re)};
+}
+
+// forward DFT-4 in place: (a,b,c,d) <- X0..X3
+__device__ __forceinline__ void dft4(Cx& a, Cx& b, Cx& c, Cx& d) {
+  const Cx p{a.re + c.re, a.im + c.im}, m{a.re - c.re, a.im - c.im};
+  const Cx q{b.re + d.re, b.im + d.im}, n{b.re - d.re, b.im - d.im};
+  a = Cx{p.re + q.re, p.im + q.im};
+  c = Cx{p.re - q.re, p.im - q.im};
+  b = Cx{m.re + n.im, m.im - n.re};
+  d = Cx{m.re - n.im, m.im + n.re};
+}
+
+// forward DFT-5 in place: (a,b,c,d,e) <- X0..X4.  With c1, c2 = cos(2 pi/5), cos(4
+// pi/5) and s1, s2 the sines: (c1 + c2)/2 = -1/4, (c1 - c2)/2 = sqrt(5)/4, s2 = 6.180339887e-01f s1
+__device__ __forceinline__ void dft5(Cx& a, Cx& b, Cx& c, Cx& d, Cx& e) {
+  constexpr float h = 5.590169944e-01f, s1 = 9.510565163e-01f, rho = 6.180339887e-01f;
+  const Cx t1{b.re + e.re, b.im + e.im}, t2{c.re + d.re, c.im + d.im};
+  const Cx t3{b.re - e.re, b.im - e.im}, t4{c.re - d.re, c.im - d.im};
+  const Cx u{t1.re + t2.re, t1.im + t2.im}, v{t1.re - t2.re, t1.im - t2.im};
+  const Cx m{fmaf(-0.25f, u.re, a.re), fmaf(-0.25f, u.im, a.im)};
+  const Cx m1{fmaf(h, v.re, m.re), fmaf(h, v.im, m.im)}, m2{fmaf(-h, v.re, m.re), fmaf(-h, v.im, m.im)};
+  const Cx n1{fmaf(rho, t4.re, t3.re), fmaf(rho, t4.im, t3.im)};
+  const Cx n2{fmaf(rho, t3.re, -t4.re), fmaf(rho, t3.im, -t4.im)};
+  a = Cx{a.re + u.re, a.im + u.im};
+  // X1 = m1 - i*s1*n1, X4 = m1 + i*s1*n1, X2 = m2 - i*s1*n2, X3 = m2 + i*s1*n2
+  b = Cx{fmaf(s1, n1.im, m1.re), fmaf(-s1, n1.re, m1.im)};
+  e = Cx{fmaf(-s1, n1.im, m1.re), fmaf(s1, n1.re, m1.im)};
+  c = Cx{fmaf(s1, n2.im, m2.re), fmaf(-s1, n2.re, m2.im)};
+  d = Cx{fmaf(-s1, n2.im, m2.re), fmaf(s1, n2.re, m2.im)};
+}
+
+// forward DFT-25 = 5 x 5; X[k1 + 5*k2] ends in v[5*k1 + k2]
+__device__ __forceinline__ void dft25(Cx (&v)[25]) {
+  dft5(v[0], v[5], v[10], v[15], v[20]);
+  dft5(v[1], v[6], v[11], v[16], v[21]);
+  dft5(v[2], v[7], v[12], v[17], v[22]);
+  dft5(v[3], v[8], v[13], v[18], v[23]);
+  dft5(v[4], v[9], v[14], v[19], v[24]);
+  cx_mul(v[6], 9.685831611e-01f, -2.486898872e-01f);  // W_25^1
+  cx_mul(v[7], 8.763066800e-01f, -4.817536741e-01f);  // W_25^2
+  cx_mul(v[8], 7.289686274e-01f, -6.845471059e-01f);  // W_25^3
+  cx_mul(v[9], 5.358267950e-01f, -8.443279255e-01f);  // W_25^4
+  cx_mul(v[11], 8.763066800e-01f, -4.817536741e-01f);  // W_25^2
+  cx_mul(v[12], 5.358267950e-01f, -8.443279255e-01f);  // W_25^4
+  cx_mul(v[13], 6.279051953e-02f, -9.980267284e-01f);  // W_25^6
+  cx_mul(v[14], -4.257792916e-01f, -9.048270525e-01f);  // W_25^8
+  cx_mul(v[16], 7.289686274e-01f, -6.845471059e-01f);  // W_25^3
+  cx_mul(v[17], 6.279051953e-02f, -9.980267284e-01f);  // W_25^6
+  cx_mul(v[18], -6.374239897e-01f, -7.705132428e-01f);  // W_25^9
+  cx_mul(v[19], -9.921147013e-01f, -1.253332336e-01f);  // W_25^12
+  cx_mul(v[21], 5.358267950e-01f, -8.443279255e-01f);  // W_25^4
+  cx_mul(v[22], -4.257792916e-01f, -9.048270525e-01f);  // W_25^8
+  cx_mul(v[23], -9.921147013e-01f, -1.253332336e-01f);  // W_25^12
+  cx_mul(v[24], -6.374239897e-01f, 7.705132428e-01f);  // W_25^16
+  dft5(v[0], v[1], v[2], v[3], v[4]);
+  dft5(v[5], v[6], v[7], v[8], v[9]);
+  dft5(v[10], v[11], v[12], v[13], v[14]);
+  dft5(v[15], v[16], v[17], v[18], v[19]);
+  dft5(v[20], v[21], v[22], v[23], v[24]);
+}
+// output index r of dft25 lives in v[dft25_pos(r)]
+__host__ __device__ constexpr int dft25_pos(int r) { return 5 * (r % 5) + r / 5; }
+
+// forward DFT-20 = 4 x 5; X[k1 + 4*k2] ends in v[5*k1 + k2]
+__device__ __forceinline__ void dft20(Cx (&v)[20]) {
+  dft4(v[0], v[5], v[10], v[15]);
+  dft4(v[1], v[6], v[11], v[16]);
+  dft4(v[2], v[7], v[12], v[17]);
+  dft4(v[3], v[8], v[13], v[18]);
+  dft4(v[4], v[9], v[14], v[19]);
+  cx_mul(v[6], 9.510565163e-01f, -3.090169944e-01f);  // W_20^1
+  cx_mul(v[7], 8.090169944e-01f, -5.877852523e-01f);  // W_20^2
+  cx_mul(v[8], 5.877852523e-01f, -8.090169944e-01f);  // W_20^3
+  cx_mul(v[9], 3.090169944e-01f, -9.510565163e-01f);  // W_20^4
+  cx_mul(v[11], 8.090169944e-01f, -5.877852523e-01f);  // W_20^2
+  cx_mul(v[12], 3.090169944e-01f, -9.510565163e-01f);  // W_20^4
+  cx_mul(v[13], -3.090169944e-01f, -9.510565163e-01f);  // W_20^6
+  cx_mul(v[14], -8.090169944e-01f, -5.877852523e-01f);  // W_20^8
+  cx_mul(v[16], 5.877852523e-01f, -8.090169944e-01f);  // W_20^3
+  cx_mul(v[17], -3.090169944e-01f, -9.510565163e-01f);  // W_20^6
+  cx_mul(v[18], -9.510565163e-01f, -3.090169944e-01f);  // W_20^9
+  cx_mul(v[19], -8.090169944e-01f, 5.877852523e-01f);  // W_20^12
+  dft5(v[0], v[1], v[2], v[3], v[4]);
+  dft5(v[5], v[6], v[7], v[8], v[9]);
+  dft5(v[10], v[11], v[12], v[13], v[14]);
+  dft5(v[15], v[16], v[17], v[18], v[19]);
+}
+// output index r of dft20 lives in v[dft20_pos(r)]
+__host__ __device__ constexpr int dft20_pos(int r) { return 5 * (r % 4) + r / 4; }
+
+}  // namespace vfrb
