@@ -18,7 +18,10 @@ constexpr int kBandSmem = 220 * 1024;     // that the tables plan for
 constexpr int kBandSmemMax = 227 * 1024;  // a CTA's limit
 constexpr int kBandMaxCh = 96;
 constexpr int kBandMax = 64;              // bands
-constexpr int kBandGeneric = 256;         // pattern code of shifts that are no staircase
+// Code of eight shifts that go up (or down) by 0 or 1 from trial to trial: bit q =
+// the step after the q-th trial, counted from the trial with shift 0; bit 7 = the
+// shifts fall (the count starts at the last trial).
+constexpr int kBandGeneric = 256;         // shifts that are no such staircase
 
 struct BandDesc {
   int c_lo, nch;    // channels [c_lo, c_lo + nch)
@@ -51,23 +54,6 @@ struct BandHost {
 
 inline long long floor_div(long long a, long long b) { return a >= 0 ? a / b : -((-a + b - 1) / b); }
 inline int floor_to(int a, int b) { return (int)floor_div(a, b) * b; }
-
-// Code of eight shifts that go up (or down) by 0 or 1 from trial to trial:
-// bit q = the step after the q-th trial, counted from the trial with shift 0;
-// bit 7 = the shifts fall (the count starts at the last trial).
-inline int band_code(const int* sh) {
-  for (int dir = 0; dir < 2; ++dir) {
-    int code = dir << 7, at = 0, q = 0;
-    for (; q < kBandD; ++q) {
-      const int v = sh[dir ? kBandD - 1 - q : q];
-      if (q && v == at + 1) code |= 1 << (q - 1);
-      else if (v != at) break;
-      at = v;
-    }
-    if (q == kBandD) return code;
-  }
-  return kBandGeneric;
-}
 
 // False when the kernel does not apply to the delay table: fewer than eight
 // trials, or trials that are not close to equally spaced.
@@ -126,23 +112,37 @@ inline bool band_build(BandHost& h, const int32_t* off, int ndm, int nchan) {
       skew[(size_t)bi * nb * G + g] = sk;
       const int32_t* r[D];
       for (int j = 0; j < D; ++j) r[j] = row(gs + j);
-      for (int c = b.c_lo; c < b.c_lo + b.nch; ++c) {
-        int v[D], mn = 0x7fffffff, mx = -0x7fffffff;
-        for (int j = 0; j < D; ++j) {
-          v[j] = r[j][c] - j * b.m;
-          mn = std::min(mn, v[j]);
-          mx = std::max(mx, v[j]);
+      const size_t i0 = (size_t)g * nchan;
+      int worst = 0;
+      unsigned odd = 0;
+      for (int c = b.c_lo; c < b.c_lo + b.nch; ++c) {  // straight-line: the compiler vectorises it
+        int v = r[0][c], mn = v, mx = v;
+        unsigned up = 0, down = 0, no_up = 0, no_down = 0;
+#pragma GCC unroll 8
+        for (int j = 1; j < D; ++j) {
+          const int n = r[j][c] - j * b.m, d = n - v;
+          v = n;
+          mn = std::min(mn, n);
+          mx = std::max(mx, n);
+          up |= (unsigned)(d & 1) << (j - 1);
+          down |= (unsigned)(d & 1) << (D - 1 - j);
+          no_up |= (unsigned)d & ~1u;
+          no_down |= (unsigned)-d & ~1u;
         }
-        if (mx - mn > kBandSmax) return false;  // not (nearly) equally spaced
-        for (int j = 0; j < D; ++j) v[j] -= mn;
-        const size_t i = (size_t)g * nchan + c;
-        base[i] = mn - sk;
-        pat[i] = (unsigned short)band_code(v);
-        if (pat[i] == kBandGeneric) {
-          if (shift.empty()) shift.assign((size_t)ng * nchan, 0u);
-          unsigned s = 0;
-          for (int j = 0; j < D; ++j) s |= (unsigned)v[j] << (4 * j);
-          shift[i] = s;
+        worst = std::max(worst, mx - mn);
+        const unsigned code = no_up == 0 ? up : no_down == 0 ? 128u | down : (unsigned)kBandGeneric;
+        odd |= code;
+        base[i0 + c] = mn - sk;
+        pat[i0 + c] = (unsigned short)code;
+      }
+      if (worst > kBandSmax) return false;  // not (nearly) equally spaced
+      if (odd & (unsigned)kBandGeneric) {
+        if (shift.empty()) shift.assign((size_t)ng * nchan, 0u);
+        for (int c = b.c_lo; c < b.c_lo + b.nch; ++c) {
+          if (pat[i0 + c] != kBandGeneric) continue;
+          unsigned sh = 0;
+          for (int j = 0; j < D; ++j) sh |= (unsigned)(r[j][c] - j * b.m - sk - base[i0 + c]) << (4 * j);
+          shift[i0 + c] = sh;
         }
       }
     }

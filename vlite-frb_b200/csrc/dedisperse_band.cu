@@ -54,6 +54,7 @@ namespace vfrb {
 
 struct BandTables {
   BandHost h;
+  unsigned char* d_all = nullptr;  // one allocation, of which the rest are parts
   int* d_bmin = nullptr;
   int* d_skew = nullptr;
   unsigned char* d_rec = nullptr;
@@ -506,10 +507,7 @@ __global__ void __launch_bounds__(kBandW * 32, 1) k_dedisp_band(const __grid_con
 // ---- host side ------------------------------------------------------------------
 void band_destroy(BandTables* t) {
   if (!t) return;
-  cudaFree(t->d_bmin);
-  cudaFree(t->d_skew);
-  cudaFree(t->d_rec);
-  cudaFree(t->d_shift);
+  cudaFree(t->d_all);
   delete t;
 }
 
@@ -518,16 +516,27 @@ int band_create(BandTables** out, const int32_t* off, int ndm, int nchan) {
   std::unique_ptr<BandTables> t(new BandTables());
   BandHost& h = t->h;
   if (!band_build(h, off, ndm, nchan)) return VFRB_OK;
-  auto up = [&](auto** d, const auto& v) {
-    if (v.empty()) return true;
-    const size_t n = v.size() * sizeof(v[0]);
-    return cudaMalloc((void**)d, n) == cudaSuccess && cudaMemcpy(*d, v.data(), n, cudaMemcpyHostToDevice) == cudaSuccess;
+  size_t used = 0;
+  auto place = [&](const auto& v) {
+    const size_t at = used;
+    used = (used + v.size() * sizeof(v[0]) + 255) / 256 * 256;
+    return at;
   };
-  if (!up(&t->d_bmin, h.bmin) || !up(&t->d_skew, h.skew) || !up(&t->d_rec, h.rec) || !up(&t->d_shift, h.shift)) {
+  const size_t at_bmin = place(h.bmin), at_skew = place(h.skew), at_rec = place(h.rec), at_shift = place(h.shift);
+  auto put = [&](size_t at, const auto& v) {
+    return v.empty() ||
+           cudaMemcpy(t->d_all + at, v.data(), v.size() * sizeof(v[0]), cudaMemcpyHostToDevice) == cudaSuccess;
+  };
+  if (cudaMalloc((void**)&t->d_all, used) != cudaSuccess || !put(at_bmin, h.bmin) || !put(at_skew, h.skew) ||
+      !put(at_rec, h.rec) || !put(at_shift, h.shift)) {
     cudaGetLastError();
     band_destroy(t.release());
     return VFRB_ERR_NOMEM;
   }
+  t->d_bmin = reinterpret_cast<int*>(t->d_all + at_bmin);
+  t->d_skew = reinterpret_cast<int*>(t->d_all + at_skew);
+  t->d_rec = t->d_all + at_rec;
+  t->d_shift = h.shift.empty() ? nullptr : reinterpret_cast<unsigned*>(t->d_all + at_shift);
   // the device has them; the launches need the bands and the skew ranges only
   h.bmin = {};
   h.skew = {};
