@@ -695,3 +695,23 @@ def test_channelise_payload_alignments(vf):
             got = vf.channelise(buf, s0, s1, sample0, rows, L, d_err=err)
             assert int(err.item()) == 0
             assert torch.equal(want.setdefault(sample0, got), got), (name, sample0)
+
+
+@pytest.mark.parametrize("ndm,nt,width", [(3, 1, 1), (5, 15, 16), (40, 1024, 256), (7, 1279, 255), (9, 4096, 64),
+                                          (4, 3000, 512)])
+def test_boxcar_tile_edges(vf, O, ndm, nt, width):
+    """Series at the tile's and the halo's edges, widths up to the tree kernel's
+    widest and one past it, pulses across tile ends, and equal samples (a tie goes
+    to the smaller width, then the earlier start)."""
+    torch = _torch()
+    rng = np.random.default_rng(nt)
+    x = np.round(rng.standard_normal((ndm, nt)) * 64).astype(np.float32) / 64  # sums are exact
+    for d in range(ndm):
+        x[d, max(0, min(nt - 1, 1000 + 9 * d)):min(nt, 1000 + 9 * d + 40)] += 2.0
+    x[0] = 0.5
+    ave = x.mean(axis=1).astype(np.float32)
+    sig = np.maximum(x.std(axis=1), 0.25).astype(np.float32)
+    best, start, w = O.boxcar_best(x, ave, sig, width)
+    snr, s0, w0 = vf.boxcar(torch.from_numpy(x).cuda(), torch.from_numpy(ave).cuda(), torch.from_numpy(sig).cuda(), width)
+    assert np.array_equal(w0.cpu().numpy(), w) and np.array_equal(s0.cpu().numpy(), start)
+    assert np.allclose(snr.cpu().numpy(), best, rtol=1e-6, atol=1e-9)

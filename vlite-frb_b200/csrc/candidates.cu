@@ -7,11 +7,12 @@
 // ave and sigma, so width 1 is calcstats' peak.  The best (snr, start,
 // width) is kept; ties go to the smaller width, then the earlier start.
 //
-// One CTA per trial; each thread slides over a contiguous stretch of the
-// series (reads are L1/L2 resident: one series is a few kB to a few hundred
-// kB), and the CTA reduces the per-thread bests.  The work is a few FP64
-// adds per sample and width: negligible next to the dedispersion that
-// produced the series.
+// One CTA per trial.  Widths up to kBoxTree: tiles of the series in shared memory,
+// where a width's sums are two of the half width's, S_2w(t) = S_w(t) + S_w(t + w):
+// one FP64 add per sample and width, and the series is read once, coalesced.  Wider
+// searches slide a window per thread over a contiguous stretch of the series, which
+// for a short series costs more in the windows' first sums (w adds for a few
+// samples per thread) than in the sliding.
 #include "vfrb_common.cuh"
 
 #include <cmath>
@@ -31,7 +32,7 @@ __device__ __forceinline__ bool box_better(const BoxBest& a, const BoxBest& b) {
   return a.t < b.t;
 }
 
-__global__ void __launch_bounds__(kBoxThreads) k_boxcar(const float* __restrict__ dd, long long nt, long long stride,
+__global__ void __launch_bounds__(kBoxThreads) k_boxcar_slide(const float* __restrict__ dd, long long nt, long long stride,
                                                          const float* __restrict__ ave, const float* __restrict__ sigma,
                                                          int max_width, float* __restrict__ snr_out,
                                                          int* __restrict__ t_out, int* __restrict__ w_out) {
@@ -70,12 +71,88 @@ __global__ void __launch_bounds__(kBoxThreads) k_boxcar(const float* __restrict_
   }
 }
 
+constexpr int kBoxTree = 256;  // widest boxcar of the tree kernel
+constexpr int kBoxTile = 1024;  // starts per tile
+constexpr int kBoxPer = kBoxTile / kBoxThreads;
+
+// WMAX: the widest boxcar, a power of two; the tile holds WMAX - 1 more samples
+__global__ void __launch_bounds__(kBoxThreads) k_boxcar_tree(const float* __restrict__ dd, long long nt,
+                                                             long long stride, const float* __restrict__ ave,
+                                                             const float* __restrict__ sigma, int wmax,
+                                                             float* __restrict__ snr_out, int* __restrict__ t_out,
+                                                             int* __restrict__ w_out) {
+  __shared__ double S[kBoxTile + kBoxTree];
+  __shared__ BoxBest red[kBoxThreads / 32];
+  const int d = blockIdx.x, tid = threadIdx.x;
+  const float* x = dd + (long long)d * stride;
+  const double a = (double)ave[d];
+  const double s = (double)sigma[d];
+  const int n = (int)nt;
+  BoxBest best{-INFINITY, 0x7fffffff, 0x7fffffff};
+  for (int t0 = 0; t0 < n; t0 += kBoxTile) {
+    // this thread's samples: tid + 256 i, the last of them in the halo
+    double v[kBoxPer + 1];
+#pragma unroll
+    for (int i = 0; i <= kBoxPer; ++i) {
+      const int p = tid + kBoxThreads * i;
+      v[i] = p < kBoxTile + wmax - 1 && t0 + p < n ? (double)x[t0 + p] : 0.0;
+    }
+    for (int w = 1;; w *= 2) {
+      const double wa = (double)w * a, inv = 1.0 / (s * sqrt((double)w));
+      const int last = n - w - t0;  // starts t0 + p <= nt - w
+#pragma unroll
+      for (int i = 0; i < kBoxPer; ++i) {
+        const int p = tid + kBoxThreads * i;
+        const double q = (v[i] - wa) * inv;
+        // ties: the smaller width (tiles are walked in time, so the earlier start of a width comes first)
+        if (p <= last && (q > best.snr || (q == best.snr && w < best.w))) best = BoxBest{q, t0 + p, w};
+      }
+      if (2 * w > wmax) break;
+      __syncthreads();  // the half width's (or the last tile's) sums have been read
+#pragma unroll
+      for (int i = 0; i <= kBoxPer; ++i) {
+        const int p = tid + kBoxThreads * i;
+        if (p < kBoxTile + kBoxTree) S[p] = v[i];
+      }
+      __syncthreads();
+#pragma unroll
+      for (int i = 0; i <= kBoxPer; ++i) {
+        const int p = tid + kBoxThreads * i;  // (what lies past the halo is not used)
+        v[i] += p + w < kBoxTile + kBoxTree ? S[p + w] : 0.0;
+      }
+    }
+  }
+  // CTA reduction with the tie rule
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    BoxBest b;
+    b.snr = __shfl_xor_sync(0xffffffffu, best.snr, o);
+    b.t = __shfl_xor_sync(0xffffffffu, best.t, o);
+    b.w = __shfl_xor_sync(0xffffffffu, best.w, o);
+    if (box_better(b, best)) best = b;
+  }
+  if ((tid & 31) == 0) red[tid >> 5] = best;
+  __syncthreads();
+  if (tid == 0) {
+    for (int q = 1; q < kBoxThreads / 32; ++q)
+      if (box_better(red[q], best)) best = red[q];
+    snr_out[d] = (float)best.snr;
+    t_out[d] = best.t;
+    w_out[d] = best.w;
+  }
+}
+
 int launch_boxcar(const float* dd, int ndm, long long nt, long long stride, const float* ave, const float* sigma,
                   int max_width, float* snr, int* t, int* w, cudaStream_t s) {
   if (!dd || !ave || !sigma || !snr || !t || !w || ndm < 1 || nt < 1 || stride < nt || max_width < 1)
     return VFRB_ERR_ARG;
   if (nt > 0x7fffffffLL) return VFRB_ERR_UNSUPPORTED;
-  k_boxcar<<<ndm, kBoxThreads, 0, s>>>(dd, nt, stride, ave, sigma, max_width, snr, t, w);
+  int wmax = 1;  // the widest width tried: powers of two up to max_width and nt
+  while (2LL * wmax <= max_width && 2LL * wmax <= nt) wmax *= 2;
+  if (wmax <= kBoxTree)
+    k_boxcar_tree<<<ndm, kBoxThreads, 0, s>>>(dd, nt, stride, ave, sigma, wmax, snr, t, w);
+  else
+    k_boxcar_slide<<<ndm, kBoxThreads, 0, s>>>(dd, nt, stride, ave, sigma, max_width, snr, t, w);
   return cuda_status(cudaGetLastError());
 }
 
