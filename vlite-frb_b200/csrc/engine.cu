@@ -182,6 +182,7 @@ struct StreamSt {
   int64_t frames_in = 0;       // frames received (ring position)
   int stash_next = 0;
   uint8_t* h_stage[kStageBufs] = {};
+  size_t stage_cap[kStageBufs] = {};  // frames each holds (made when first needed)
   // device input: each batch's 32-byte frame headers, packed in
   // page-locked host memory by one strided copy
   uint8_t* h_hdr = nullptr;
@@ -993,6 +994,17 @@ int64_t oldest_ref(const StreamSt* s) {
   return o;
 }
 
+// Staging buffer k holds at least nb frames.  A frame that straddles pushes comes
+// alone: a small buffer for those, the whole one when a longer run comes.  (The
+// buffer it replaces stays with the stream: copies from it may be in flight.)
+int stage_buffer(StreamSt* s, int k, size_t nb) {
+  if (s->stage_cap[k] >= nb) return VFRB_OK;
+  const size_t cap = nb <= 16 ? 16 : s->stage_frames;
+  ST(hmalloc(s->res, &s->h_stage[k], std::max(cap, nb) * kFrameLen));
+  s->stage_cap[k] = std::max(cap, nb);
+  return VFRB_OK;
+}
+
 // Copy `nf` whole frames to the ring, queue their headers, advance.
 int feed_frames(vfrb_plan* pl, StreamSt* s, const uint8_t* in, int64_t nf, MemKind kind) {
   const Range nvtx_range("vfrb feed frames");
@@ -1050,6 +1062,9 @@ int feed_frames(vfrb_plan* pl, StreamSt* s, const uint8_t* in, int64_t nf, MemKi
       const int k = s->stage_i;
       s->stage_i = (s->stage_i + 1) % kStageBufs;
       CK(cudaEventSynchronize(s->stage_ev[k]));
+      // page-locking these (up to 41 MB each) is most of a stream's opening: they
+      // are made when pageable input first needs one of its size
+      ST(stage_buffer(s, k, (size_t)nb));
       std::memcpy(s->h_stage[k], src, (size_t)nb * kFrameLen);
       from = s->h_stage[k];
       // the staging event is recorded after the copies below
@@ -1135,7 +1150,6 @@ int create_stream(vfrb_plan* pl, int id, int64_t ring_frames, int64_t R1, int64_
   s->stage_frames = (size_t)std::min<int64_t>(ring_frames / 4, 8192);
   ST(hmalloc(s->res, &s->h_hdr, (size_t)std::max<int64_t>(1, ring_frames / 4) * kHdrLen));
   for (int k = 0; k < kStageBufs; ++k) {
-    ST(hmalloc(s->res, &s->h_stage[k], s->stage_frames * kFrameLen));
     ST(mkevent(s->res, &s->stage_ev[k]));
     CK(cudaEventRecord(s->stage_ev[k], s->xs));
   }
