@@ -109,13 +109,11 @@ __device__ __forceinline__ void bp_window(const vfrb_bp_args& a, __half* __restr
     float* row = tile[cl] + g;
     double cave = 0.0, sig = 0.0;  // subtract_mode 1: copy only (cave = 0)
     if (a.subtract_mode == 0) {
-      float x[kRows];
       double xd[kRows];
       double s = 0.0;
 #pragma unroll
       for (int k = 0; k < kRows; ++k) {
-        x[k] = row[8 * k];  // rows past the window hold zeros
-        xd[k] = (double)x[k];
+        xd[k] = (double)row[8 * k];  // rows past the window hold zeros
         s += xd[k];
       }
       const double n = (double)npts;
@@ -133,19 +131,18 @@ __device__ __forceinline__ void bp_window(const vfrb_bp_args& a, __half* __restr
       sd = sum8(sd);
       sd2 = sum8(sd2);
       sig = (sd2 - (sd * sd) / n) / (n - 1.0);  // variance, NaN when npts == 1
-      // the clip decided in FP32: the thresholds rounded outwards order every float alike
-      const float hi = __double2float_ru(ave + 3.0 * sig), lo = __double2float_rd(ave - 3.0 * sig);
+      const double hi = ave + 3.0 * sig, lo = ave - 3.0 * sig;
       bool all = true;
 #pragma unroll
       for (int k = 0; k < kRows; ++k)
-        if (FULL || g + 8 * k < npts) all = all && x[k] < hi && x[k] > lo;
+        if (FULL || g + 8 * k < npts) all = all && xd[k] < hi && xd[k] > lo;
       double cnt = n, cs = s;
       if (!__all_sync(0xffffffffu, all)) {  // some channel of the warp loses rows
         int kept = 0;
         cs = 0.0;
 #pragma unroll
         for (int k = 0; k < kRows; ++k)
-          if ((FULL || g + 8 * k < npts) && x[k] < hi && x[k] > lo) {
+          if ((FULL || g + 8 * k < npts) && xd[k] < hi && xd[k] > lo) {
             cs += xd[k];
             ++kept;
           }
@@ -225,7 +222,9 @@ __device__ __forceinline__ void bp_window(const vfrb_bp_args& a, __half* __restr
 }
 
 template <int STORAGE>
-__global__ void __launch_bounds__(kBpThreads) k_bandpass(const __grid_constant__ vfrb_bp_args a,
+// (four CTAs per SM: 64 registers; 92 us at 7680 x 6250, with three 100, with five,
+// which spills, 102)
+__global__ void __launch_bounds__(kBpThreads, 4) k_bandpass(const __grid_constant__ vfrb_bp_args a,
                                                          __half* __restrict__ out1) {
   __shared__ float tile[kBpChan][kBpMaxWin + 1];
   const bool full = a.window == kBpMaxWin && (long long)(blockIdx.y + 1) * kBpMaxWin <= a.nrows &&
