@@ -29,10 +29,19 @@
 // ones of warps 0 to 3 run meanwhile.  (Payloads are 8 mod 16 apart, so no shift of
 // the window makes all its pieces legal 16-byte or bulk copies.)
 //
+// What bounds it: instruction issue (70% of the slots; FMA pipe 51%, shared memory 50%
+// of the wavefronts), with the slots that stay empty at the start of each pass, where
+// loads come faster than they are served.  8192 rows x 10 windows: 4.33 ms -> 3.53 ms.
+// On the way: the transform alone 4.26, its passes in place 4.05, threads mapped so
+// that half warps touch different banks 3.75, 8-byte staging copies 3.64, loads
+// interleaved with the inner DFTs 3.53.  A second Z, which saves a barrier per window
+// but leaves room for one staging buffer only: 3.59.
+//
 // Few rows: a row's NAVE windows are one after another in a CTA, so a 32-row bundle
 // would use 32 SMs.  Where all windows of a call fit the device at once, a cluster of
 // NAVE CTAs takes a row, one window each, and adds the powers in window order
-// through distributed shared memory: the same sums bit for bit.
+// through distributed shared memory: the same sums bit for bit.  A 32-row bundle of 4
+// windows: 36.9 -> 14.4 us.
 #include "vfrb_common.cuh"
 #include "dft_codelets.cuh"
 
@@ -41,6 +50,7 @@
 #include <algorithm>
 #include <cmath>
 #include <mutex>
+#include <type_traits>
 
 namespace cg = cooperative_groups;
 
@@ -116,6 +126,23 @@ static int ensure_twiddles() {
 
 __device__ __forceinline__ void cp_async_commit_k1() { asm volatile("cp.async.commit_group;\n" ::); }
 __device__ __forceinline__ void cp_async_wait_k1() { asm volatile("cp.async.wait_group 0;\n" ::: "memory"); }
+
+// f(0), ..., f(4) with compile-time arguments.  A butterfly's inner DFTs take every
+// fifth input: each group of loads is followed by its arithmetic and kept there (the
+// empty asm), so that a warp computes while the others' loads are served, where all
+// loads first would leave the arithmetic idle until the last one.
+template <typename F>
+__device__ __forceinline__ void each5(F&& f) {
+  f(std::integral_constant<int, 0>{});
+  asm volatile("" ::: "memory");
+  f(std::integral_constant<int, 1>{});
+  asm volatile("" ::: "memory");
+  f(std::integral_constant<int, 2>{});
+  asm volatile("" ::: "memory");
+  f(std::integral_constant<int, 3>{});
+  asm volatile("" ::: "memory");
+  f(std::integral_constant<int, 4>{});
+}
 
 // byte b as the float b - 128, exactly: 0x4B0000bb is the float 2^23 + b
 __device__ __forceinline__ float centred(unsigned b) { return __uint_as_float(0x4B000000u | b) - 8388736.0f; }
@@ -273,9 +300,13 @@ __global__ void __launch_bounds__(kThreads, 1) k_channelise(const __grid_constan
     // pass 1: R = 20, Ns = 1, from the staged bytes
     for (int j = tid; j < kB1; j += kThreads) {
       Cx v[20];
+      each5([&](auto q) {
+        constexpr int Q = decltype(q)::value;
 #pragma unroll
-      for (int r = 0; r < 20; ++r) v[r] = Cx{centred(x0[j + kB1 * r]), centred(x1[j + kB1 * r])};
-      dft20(v);
+        for (int r = Q; r < 20; r += 5) v[r] = Cx{centred(x0[j + kB1 * r]), centred(x1[j + kB1 * r])};
+        dft20_inner<Q>(v);
+      });
+      dft20_outer(v);
 #pragma unroll
       for (int k = 0; k < 20; ++k) Z[j + kB1 * k] = make_float2(v[dft20_pos(k)].re, v[dft20_pos(k)].im);
     }
@@ -284,18 +315,21 @@ __global__ void __launch_bounds__(kThreads, 1) k_channelise(const __grid_constan
     Cx v[25];
     if (tid < kB) {
       float2* io = Z + g + kB1 * m;
-#pragma unroll
-      for (int r = 0; r < 25; ++r) {
-        const float2 q = io[25 * r];
-        v[r] = Cx{q.x, q.y};
-      }
       const float2* tw = tw2 + m + z;
+      each5([&](auto q) {
+        constexpr int Q = decltype(q)::value;
 #pragma unroll
-      for (int r = 1; r < 25; ++r) {
-        const float2 t = tw[(r - 1) * 20];
-        cx_mul(v[r], t.x, t.y);
-      }
-      dft25(v);
+        for (int r = Q; r < 25; r += 5) {
+          const float2 x = io[25 * r];
+          v[r] = Cx{x.x, x.y};
+          if (r) {
+            const float2 t = tw[(r - 1) * 20];
+            cx_mul(v[r], t.x, t.y);
+          }
+        }
+        dft25_inner<Q>(v);
+      });
+      dft25_outer(v);
 #pragma unroll
       for (int k = 0; k < 25; ++k) io[25 * k] = make_float2(v[dft25_pos(k)].re, v[dft25_pos(k)].im);
     }
@@ -331,7 +365,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_channelise(const __grid_constan
           cx_mul(v[5 * q + i], p.re, p.im);
         }
       }
-      dft25(v);
+      each5([&](auto q) { dft25_inner<decltype(q)::value>(v); });
+      dft25_outer(v);
 #pragma unroll
       for (int k = 0; k < 25; ++k) {
         const Cx x = v[dft25_pos(k)];

@@ -48,29 +48,37 @@ __device__ __forceinline__ void dft5(Cx& a, Cx& b, Cx& c, Cx& d, Cx& e) {
   d = Cx{fmaf(-s1, n2.im, m2.re), fmaf(s1, n2.re, m2.im)};
 }
 
-// forward DFT-25 = 5 x 5; X[k1 + 5*k2] ends in v[5*k1 + k2]
-__device__ __forceinline__ void dft25(Cx (&v)[25]) {
-  dft5(v[0], v[5], v[10], v[15], v[20]);
-  dft5(v[1], v[6], v[11], v[16], v[21]);
-  dft5(v[2], v[7], v[12], v[17], v[22]);
-  dft5(v[3], v[8], v[13], v[18], v[23]);
-  dft5(v[4], v[9], v[14], v[19], v[24]);
-  cx_mul(v[6], 9.685831611e-01f, -2.486898872e-01f);  // W_25^1
-  cx_mul(v[7], 8.763066800e-01f, -4.817536741e-01f);  // W_25^2
-  cx_mul(v[8], 7.289686274e-01f, -6.845471059e-01f);  // W_25^3
-  cx_mul(v[9], 5.358267950e-01f, -8.443279255e-01f);  // W_25^4
-  cx_mul(v[11], 8.763066800e-01f, -4.817536741e-01f);  // W_25^2
-  cx_mul(v[12], 5.358267950e-01f, -8.443279255e-01f);  // W_25^4
-  cx_mul(v[13], 6.279051953e-02f, -9.980267284e-01f);  // W_25^6
-  cx_mul(v[14], -4.257792916e-01f, -9.048270525e-01f);  // W_25^8
-  cx_mul(v[16], 7.289686274e-01f, -6.845471059e-01f);  // W_25^3
-  cx_mul(v[17], 6.279051953e-02f, -9.980267284e-01f);  // W_25^6
-  cx_mul(v[18], -6.374239897e-01f, -7.705132428e-01f);  // W_25^9
-  cx_mul(v[19], -9.921147013e-01f, -1.253332336e-01f);  // W_25^12
-  cx_mul(v[21], 5.358267950e-01f, -8.443279255e-01f);  // W_25^4
-  cx_mul(v[22], -4.257792916e-01f, -9.048270525e-01f);  // W_25^8
-  cx_mul(v[23], -9.921147013e-01f, -1.253332336e-01f);  // W_25^12
-  cx_mul(v[24], -6.374239897e-01f, 7.705132428e-01f);  // W_25^16
+// forward DFT-25 = 5 x 5; X[k1 + 5*k2] ends in v[5*k1 + k2].  The inner DFT of
+// inputs Q, Q + 5, ... and its twiddles (for each Q < 5), then the outer ones:
+template <int Q>
+__device__ __forceinline__ void dft25_inner(Cx (&v)[25]) {
+  dft5(v[Q + 0], v[Q + 5], v[Q + 10], v[Q + 15], v[Q + 20]);
+  if constexpr (Q == 1) {
+    cx_mul(v[6], 9.685831611e-01f, -2.486898872e-01f);  // W_25^1
+    cx_mul(v[11], 8.763066800e-01f, -4.817536741e-01f);  // W_25^2
+    cx_mul(v[16], 7.289686274e-01f, -6.845471059e-01f);  // W_25^3
+    cx_mul(v[21], 5.358267950e-01f, -8.443279255e-01f);  // W_25^4
+  }
+  if constexpr (Q == 2) {
+    cx_mul(v[7], 8.763066800e-01f, -4.817536741e-01f);  // W_25^2
+    cx_mul(v[12], 5.358267950e-01f, -8.443279255e-01f);  // W_25^4
+    cx_mul(v[17], 6.279051953e-02f, -9.980267284e-01f);  // W_25^6
+    cx_mul(v[22], -4.257792916e-01f, -9.048270525e-01f);  // W_25^8
+  }
+  if constexpr (Q == 3) {
+    cx_mul(v[8], 7.289686274e-01f, -6.845471059e-01f);  // W_25^3
+    cx_mul(v[13], 6.279051953e-02f, -9.980267284e-01f);  // W_25^6
+    cx_mul(v[18], -6.374239897e-01f, -7.705132428e-01f);  // W_25^9
+    cx_mul(v[23], -9.921147013e-01f, -1.253332336e-01f);  // W_25^12
+  }
+  if constexpr (Q == 4) {
+    cx_mul(v[9], 5.358267950e-01f, -8.443279255e-01f);  // W_25^4
+    cx_mul(v[14], -4.257792916e-01f, -9.048270525e-01f);  // W_25^8
+    cx_mul(v[19], -9.921147013e-01f, -1.253332336e-01f);  // W_25^12
+    cx_mul(v[24], -6.374239897e-01f, 7.705132428e-01f);  // W_25^16
+  }
+}
+__device__ __forceinline__ void dft25_outer(Cx (&v)[25]) {
   dft5(v[0], v[1], v[2], v[3], v[4]);
   dft5(v[5], v[6], v[7], v[8], v[9]);
   dft5(v[10], v[11], v[12], v[13], v[14]);
@@ -80,25 +88,33 @@ __device__ __forceinline__ void dft25(Cx (&v)[25]) {
 // output index r of dft25 lives in v[dft25_pos(r)]
 __host__ __device__ constexpr int dft25_pos(int r) { return 5 * (r % 5) + r / 5; }
 
-// forward DFT-20 = 4 x 5; X[k1 + 4*k2] ends in v[5*k1 + k2]
-__device__ __forceinline__ void dft20(Cx (&v)[20]) {
-  dft4(v[0], v[5], v[10], v[15]);
-  dft4(v[1], v[6], v[11], v[16]);
-  dft4(v[2], v[7], v[12], v[17]);
-  dft4(v[3], v[8], v[13], v[18]);
-  dft4(v[4], v[9], v[14], v[19]);
-  cx_mul(v[6], 9.510565163e-01f, -3.090169944e-01f);  // W_20^1
-  cx_mul(v[7], 8.090169944e-01f, -5.877852523e-01f);  // W_20^2
-  cx_mul(v[8], 5.877852523e-01f, -8.090169944e-01f);  // W_20^3
-  cx_mul(v[9], 3.090169944e-01f, -9.510565163e-01f);  // W_20^4
-  cx_mul(v[11], 8.090169944e-01f, -5.877852523e-01f);  // W_20^2
-  cx_mul(v[12], 3.090169944e-01f, -9.510565163e-01f);  // W_20^4
-  cx_mul(v[13], -3.090169944e-01f, -9.510565163e-01f);  // W_20^6
-  cx_mul(v[14], -8.090169944e-01f, -5.877852523e-01f);  // W_20^8
-  cx_mul(v[16], 5.877852523e-01f, -8.090169944e-01f);  // W_20^3
-  cx_mul(v[17], -3.090169944e-01f, -9.510565163e-01f);  // W_20^6
-  cx_mul(v[18], -9.510565163e-01f, -3.090169944e-01f);  // W_20^9
-  cx_mul(v[19], -8.090169944e-01f, 5.877852523e-01f);  // W_20^12
+// forward DFT-20 = 4 x 5; X[k1 + 4*k2] ends in v[5*k1 + k2].  The inner DFT of
+// inputs Q, Q + 5, ... and its twiddles (for each Q < 5), then the outer ones:
+template <int Q>
+__device__ __forceinline__ void dft20_inner(Cx (&v)[20]) {
+  dft4(v[Q + 0], v[Q + 5], v[Q + 10], v[Q + 15]);
+  if constexpr (Q == 1) {
+    cx_mul(v[6], 9.510565163e-01f, -3.090169944e-01f);  // W_20^1
+    cx_mul(v[11], 8.090169944e-01f, -5.877852523e-01f);  // W_20^2
+    cx_mul(v[16], 5.877852523e-01f, -8.090169944e-01f);  // W_20^3
+  }
+  if constexpr (Q == 2) {
+    cx_mul(v[7], 8.090169944e-01f, -5.877852523e-01f);  // W_20^2
+    cx_mul(v[12], 3.090169944e-01f, -9.510565163e-01f);  // W_20^4
+    cx_mul(v[17], -3.090169944e-01f, -9.510565163e-01f);  // W_20^6
+  }
+  if constexpr (Q == 3) {
+    cx_mul(v[8], 5.877852523e-01f, -8.090169944e-01f);  // W_20^3
+    cx_mul(v[13], -3.090169944e-01f, -9.510565163e-01f);  // W_20^6
+    cx_mul(v[18], -9.510565163e-01f, -3.090169944e-01f);  // W_20^9
+  }
+  if constexpr (Q == 4) {
+    cx_mul(v[9], 3.090169944e-01f, -9.510565163e-01f);  // W_20^4
+    cx_mul(v[14], -8.090169944e-01f, -5.877852523e-01f);  // W_20^8
+    cx_mul(v[19], -8.090169944e-01f, 5.877852523e-01f);  // W_20^12
+  }
+}
+__device__ __forceinline__ void dft20_outer(Cx (&v)[20]) {
   dft5(v[0], v[1], v[2], v[3], v[4]);
   dft5(v[5], v[6], v[7], v[8], v[9]);
   dft5(v[10], v[11], v[12], v[13], v[14]);

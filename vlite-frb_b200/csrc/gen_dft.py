@@ -78,16 +78,19 @@ __device__ __forceinline__ void dft5(Cx& a, Cx& b, Cx& c, Cx& d, Cx& e) {
 
 def codelet(n1: int, n2: int) -> str:
     n = n1 * n2
-    s = f"\n// forward DFT-{n} = {n1} x {n2}; X[k1 + {n1}*k2] ends in v[{n2}*k1 + k2]\n"
-    s += f"__device__ __forceinline__ void dft{n}(Cx (&v)[{n}]) {{\n"
-    for q in range(n2):
-        s += f"  dft{n1}({', '.join(f'v[{n2 * i + q}]' for i in range(n1))});\n"
-    for k1 in range(n1):
-        for q in range(n2):
-            e = (q * k1) % n
-            if e:
-                c, sn = w(e, n)
-                s += f"  cx_mul(v[{n2 * k1 + q}], {lit(c)}, {lit(sn)});  // W_{n}^{e}\n"
+    s = f"\n// forward DFT-{n} = {n1} x {n2}; X[k1 + {n1}*k2] ends in v[{n2}*k1 + k2].  The inner DFT of\n"
+    s += f"// inputs Q, Q + {n2}, ... and its twiddles (for each Q < {n2}), then the outer ones:\n"
+    s += "template <int Q>\n"
+    s += f"__device__ __forceinline__ void dft{n}_inner(Cx (&v)[{n}]) {{\n"
+    s += f"  dft{n1}({', '.join(f'v[Q + {n2 * i}]' for i in range(n1))});\n"
+    for q in range(1, n2):
+        s += f"  if constexpr (Q == {q}) {{\n"
+        for k1 in range(1, n1):
+            c, sn = w((q * k1) % n, n)
+            s += f"    cx_mul(v[{n2 * k1 + q}], {lit(c)}, {lit(sn)});  // W_{n}^{(q * k1) % n}\n"
+        s += "  }\n"
+    s += "}\n"
+    s += f"__device__ __forceinline__ void dft{n}_outer(Cx (&v)[{n}]) {{\n"
     for k1 in range(n1):
         s += f"  dft{n2}({', '.join(f'v[{n2 * k1 + q}]' for q in range(n2))});\n"
     s += "}\n"
