@@ -29,13 +29,14 @@
 // ones of warps 0 to 3 run meanwhile.  (Payloads are 8 mod 16 apart, so no shift of
 // the window makes all its pieces legal 16-byte or bulk copies.)
 //
-// What bounds it: instruction issue (70% of the slots; FMA pipe 51%, shared memory 50%
+// What bounds it: instruction issue (62% of the slots; FMA pipe 54%, shared memory 50%
 // of the wavefronts), with the slots that stay empty at the start of each pass, where
-// loads come faster than they are served.  8192 rows x 10 windows: 4.33 ms -> 3.53 ms.
+// loads come faster than they are served.  8192 rows x 10 windows: 4.33 ms -> 3.46 ms.
 // On the way: the transform alone 4.26, its passes in place 4.05, threads mapped so
 // that half warps touch different banks 3.75, 8-byte staging copies 3.64, loads
-// interleaved with the inner DFTs 3.53.  A second Z, which saves a barrier per window
-// but leaves room for one staging buffer only: 3.59.
+// interleaved with the inner DFTs 3.53, packed adds and FMAs for (re, im) in the DFT-4
+// and DFT-5 (14% fewer instructions) 3.46.  A second Z, which saves a barrier per
+// window but leaves room for one staging buffer only: 3.70.
 //
 // Few rows: a row's NAVE windows are one after another in a CTA, so a 32-row bundle
 // would use 32 SMs.  Where all windows of a call fit the device at once, a cluster of

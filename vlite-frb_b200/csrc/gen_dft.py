@@ -45,33 +45,47 @@ __device__ __forceinline__ Cx cx_prod(Cx a, Cx b) {
   return Cx{fmaf(-a.im, b.im, a.re * b.re), fmaf(a.re, b.im, a.im * b.re)};
 }
 
+// packed pairs (re, im): one instruction for both where nothing crosses over
+__device__ __forceinline__ float2 f2(const Cx& v) { return make_float2(v.re, v.im); }
+__device__ __forceinline__ float2 f2s(float c) { return make_float2(c, c); }
+__device__ __forceinline__ float2 f2subv(float2 a, float2 b) {
+  unsigned long long x, y, d;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(x) : "f"(a.x), "f"(a.y));
+  asm("mov.b64 %0, {%1, %2};" : "=l"(y) : "f"(b.x), "f"(b.y));
+  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(x), "l"(y));
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(d));
+  return r;
+}
+__device__ __forceinline__ float2 f2add(const Cx& a, const Cx& b) { return __fadd2_rn(f2(a), f2(b)); }
+__device__ __forceinline__ float2 f2sub(const Cx& a, const Cx& b) { return f2subv(f2(a), f2(b)); }
+
 // forward DFT-4 in place: (a,b,c,d) <- X0..X3
 __device__ __forceinline__ void dft4(Cx& a, Cx& b, Cx& c, Cx& d) {
-  const Cx p{a.re + c.re, a.im + c.im}, m{a.re - c.re, a.im - c.im};
-  const Cx q{b.re + d.re, b.im + d.im}, n{b.re - d.re, b.im - d.im};
-  a = Cx{p.re + q.re, p.im + q.im};
-  c = Cx{p.re - q.re, p.im - q.im};
-  b = Cx{m.re + n.im, m.im - n.re};
-  d = Cx{m.re - n.im, m.im + n.re};
+  const float2 p = f2add(a, c), m = f2sub(a, c), q = f2add(b, d), n = f2sub(b, d);
+  const float2 x0 = __fadd2_rn(p, q), x2 = f2subv(p, q);
+  a = Cx{x0.x, x0.y};
+  c = Cx{x2.x, x2.y};
+  b = Cx{m.x + n.y, m.y - n.x};
+  d = Cx{m.x - n.y, m.y + n.x};
 }
 
 // forward DFT-5 in place: (a,b,c,d,e) <- X0..X4.  With c1, c2 = cos(2 pi/5), cos(4
 // pi/5) and s1, s2 the sines: (c1 + c2)/2 = -1/4, (c1 - c2)/2 = sqrt(5)/4, s2 = RHO s1
 __device__ __forceinline__ void dft5(Cx& a, Cx& b, Cx& c, Cx& d, Cx& e) {
   constexpr float h = H5, s1 = S1, rho = RHO;
-  const Cx t1{b.re + e.re, b.im + e.im}, t2{c.re + d.re, c.im + d.im};
-  const Cx t3{b.re - e.re, b.im - e.im}, t4{c.re - d.re, c.im - d.im};
-  const Cx u{t1.re + t2.re, t1.im + t2.im}, v{t1.re - t2.re, t1.im - t2.im};
-  const Cx m{fmaf(-0.25f, u.re, a.re), fmaf(-0.25f, u.im, a.im)};
-  const Cx m1{fmaf(h, v.re, m.re), fmaf(h, v.im, m.im)}, m2{fmaf(-h, v.re, m.re), fmaf(-h, v.im, m.im)};
-  const Cx n1{fmaf(rho, t4.re, t3.re), fmaf(rho, t4.im, t3.im)};
-  const Cx n2{fmaf(rho, t3.re, -t4.re), fmaf(rho, t3.im, -t4.im)};
-  a = Cx{a.re + u.re, a.im + u.im};
+  const float2 t1 = f2add(b, e), t2 = f2add(c, d), t3 = f2sub(b, e), t4 = f2sub(d, c);  // t4 negated
+  const float2 u = __fadd2_rn(t1, t2), m = __ffma2_rn(f2s(-0.25f), u, f2(a));
+  const float2 v = f2subv(t1, t2);
+  const float2 m1 = __ffma2_rn(f2s(h), v, m), m2 = __ffma2_rn(f2s(-h), v, m);
+  const float2 n1 = __ffma2_rn(f2s(-rho), t4, t3), n2 = __ffma2_rn(f2s(rho), t3, t4);
+  const float2 a0 = __fadd2_rn(f2(a), u);
+  a = Cx{a0.x, a0.y};
   // X1 = m1 - i*s1*n1, X4 = m1 + i*s1*n1, X2 = m2 - i*s1*n2, X3 = m2 + i*s1*n2
-  b = Cx{fmaf(s1, n1.im, m1.re), fmaf(-s1, n1.re, m1.im)};
-  e = Cx{fmaf(-s1, n1.im, m1.re), fmaf(s1, n1.re, m1.im)};
-  c = Cx{fmaf(s1, n2.im, m2.re), fmaf(-s1, n2.re, m2.im)};
-  d = Cx{fmaf(-s1, n2.im, m2.re), fmaf(s1, n2.re, m2.im)};
+  b = Cx{fmaf(s1, n1.y, m1.x), fmaf(-s1, n1.x, m1.y)};
+  e = Cx{fmaf(-s1, n1.y, m1.x), fmaf(s1, n1.x, m1.y)};
+  c = Cx{fmaf(s1, n2.y, m2.x), fmaf(-s1, n2.x, m2.y)};
+  d = Cx{fmaf(-s1, n2.y, m2.x), fmaf(s1, n2.x, m2.y)};
 }
 """
 
