@@ -236,8 +236,10 @@ def run_device(vf, frames, storage, steps, warmup, dist, variant=0):
     ms = dist_max(dist, ms)
     stage /= steps
     return dict(ms=ms, stage_ms=stage.tolist(), rows=pipe.rows, md=pipe.md, clocks=clk.summary(),
-                stats=pipe.stats, nchan=pipe.L.nchanout, launches=4, tune=pipe.tune,
-                variant=pipe.plan.variant(storage))
+                stats=pipe.stats, nchan=pipe.L.nchanout,
+                # K1, K2, then seven bands + k_series_part + k_dm_stats, or one pinned kernel + k_dm_stats
+                launches=4 if variant else 11, tune=pipe.tune,
+                variant=pipe.plan.variant(storage) if variant else "auto (band-wise)")
 
 
 # --------------------------------------------------------------------------- e2e through the plan API

@@ -8,9 +8,9 @@
 // whole number m.  Within it trial j of a group is accumulated m*j rows
 // earlier, so the eight delays differ by a digital straight line of slope
 // y_c - m, at most 1/2 row per trial: they span at most 4 rows, and there are
-// only 67 such patterns, 8 or 9 of which occur among 60 neighbouring channels.  Channels with the same pattern are summed FIRST, one
-// add per window element, and their sum is then added to the eight trials at
-// the pattern's eight shifts.  Every series is the sum of exactly the
+// only 67 such patterns, 8 or 9 of which occur among 60 neighbouring channels.
+// Channels with the same pattern are summed FIRST, one add per window element, and
+// their sum is then added to the eight trials at the pattern's eight shifts.  Every series is the sum of exactly the
 // samples that the brute-force sum takes; only the order of the FP32 additions
 // differs, and it is shorter (runs of a few channels, then chunks, then bands),
 // which lowers the rounding error.
@@ -24,9 +24,9 @@
 // kernel) -> 6.6 ms; 2048 x 1024 in FP16 1.50 -> 0.78 ms; 201 trials x 5145
 // samples 1.65 -> 0.59 ms, in int8 2.37 (staged kernel) -> 0.84 ms.  Longer runs
 // per lane with fewer warps have fewer loads and instructions per sum but were no
-// faster: TT 15 with 12 warps 8.0 ms, with 8 warps 8.1 ms, where this shape took
-// 7.2 (all before bands overlapped); TT 7 x 20 warps 7.2 ms.  Two 8-warp CTAs per
-// SM hold half as many channels per chunk, so runs are shorter: 8.1 ms.
+// faster: TT 11 with 12 warps 7.0 ms, TT 17 with 8 warps 8.5 ms; nor were more
+// warps with shorter runs, TT 7 x 20 warps 7.3 ms.  Two 8-warp CTAs per SM hold
+// half as many channels per chunk, so runs are shorter: 8.1 ms.
 //
 // Each band is a launch of its own: trial d's accumulators cover the samples
 // t = t' - skew(d, band) of a tile [t0, t0 + NT) of t', skew being the delay of

@@ -231,8 +231,9 @@ struct StreamSt {
   // both
   void* d_cm = nullptr;  // channel-major bandpassed FB (storage form)
   // FP16 with dedispersion: the same ring shifted by one row,
-  // d_cm1[c][r] = d_cm[c][r + 1] (written by the bandpass beside d_cm), so
-  // the dedisperser reads its windows of halves with aligned 4-byte loads
+  // d_cm1[c][r] = d_cm[c][r + 1] (written by the bandpass beside d_cm), so the
+  // four-trial pattern kernel, which takes trial lists that are not equally
+  // spaced, reads its windows of halves with aligned 4-byte loads
   void* d_cm1 = nullptr;
   int64_t cm_stride = 0;
   unsigned cm_mask = 0xffffffffu;
