@@ -715,3 +715,25 @@ def test_boxcar_tile_edges(vf, O, ndm, nt, width):
     snr, s0, w0 = vf.boxcar(torch.from_numpy(x).cuda(), torch.from_numpy(ave).cuda(), torch.from_numpy(sig).cuda(), width)
     assert np.array_equal(w0.cpu().numpy(), w) and np.array_equal(s0.cpu().numpy(), start)
     assert np.allclose(snr.cpu().numpy(), best, rtol=1e-6, atol=1e-9)
+
+
+@pytest.mark.parametrize("nch,rows,row0,ring", [(50, 300, 450, 512), (1664, 37, 0, 40), (1665, 37, 508, 512),
+                                                (6250, 61, 3, 64), (6251, 30, 4, 64), (56001, 9, 0, 12), (57000, 9, 0, 12)])
+def test_subtract_zero_slices(vf, O, nch, rows, row0, ring):
+    """subtractZERO with one to eight slices of the channels, aligned and
+    unaligned rows, a ragged last group and a wrapped ring, within one float
+    rounding of the FP64 oracle; other rows stay as they are."""
+    torch = _torch()
+    x = _rfi_fb(rows, nch, seed=nch)
+    wrap = ring & (ring - 1) == 0
+    idx = (row0 + np.arange(rows)) % ring if wrap else row0 + np.arange(rows)
+    buf = np.full((nch, ring), 7.0, np.float32)
+    buf[:, idx] = x.T
+    cm = torch.from_numpy(buf).cuda()
+    kw = dict(row_mask=ring - 1) if wrap else {}
+    vf.subtract_zero(cm, nrows=rows, row0=row0, **kw)
+    got = cm.cpu().numpy()
+    ref = O.subtract_zero(x.astype(np.float64))
+    assert np.max(np.abs(got[:, idx].T - ref)) <= 1e-6 * np.abs(x).max()
+    rest = np.setdiff1d(np.arange(ring), idx)
+    assert (got[:, rest] == 7.0).all()

@@ -19,9 +19,14 @@
 // through memory four times.
 #include "vfrb_common.cuh"
 
+#include <cooperative_groups.h>
+
 #include <algorithm>
 
+namespace cg = cooperative_groups;
+
 namespace vfrb {
+
 
 __device__ __forceinline__ double rfi_wsum(double v) {
 #pragma unroll
@@ -122,98 +127,189 @@ __global__ void __launch_bounds__(256) k_subtract_bp_full(float* __restrict__ fb
 }
 
 // ---- zero-DM ----------------------------------------------------------------------
-// A CTA takes 8 consecutive rows of every channel: 32-byte runs, a whole sector of
-// memory each, into shared memory (200 kB at 6250 channels) with asynchronous
-// copies.  Thread t has row t % 8 and every 64th channel, so a warp's shared
-// accesses are 32 consecutive words.  The clipped mean of a row that loses nothing
-// to the clip is its sum, so the third pass only compares, in FP32.  7680 rows x
-// 6250 channels: 4.99 ms with a thread per row and four passes over memory (30
-// CTAs), 0.21 ms.  Clusters of eight CTAs with 32-row tiles (full 128-byte lines,
-// two CTAs per SM) took 0.23 ms.
+// A cluster of CTAs takes 8 consecutive rows of every channel, 32-byte runs (a whole
+// sector of memory each), a slice of the channels per CTA, into shared memory with
+// asynchronous copies.  A thread has four rows of every (kZeroThreads / 2)-th channel:
+// 16-byte copies and accesses where the rows are aligned.  The slices' row sums are
+// added in rank order through distributed shared memory.
+//
+// Slices of up to 52 kB let four CTAs share an SM, so that one's copies run beside
+// another's sums.  Bound by the latency of the three reductions and of the FP64
+// sums; 384 MB at 2.9 TB/s.  7680 rows x 6250 channels: 4.99 ms with a thread per row
+// and four passes over memory (30 CTAs); 0.209 ms with one CTA of 200 kB for all
+// channels and 4-byte accesses; 0.147 ms with four slices; 0.134 ms with the
+// divisions in one thread per row and reductions that halve the values at each step.
+// Two slices of 512 threads 0.146 ms; eight of 128 threads 0.131 ms, not worth the
+// larger clusters.
 constexpr int kZeroRows = 8;
-constexpr int kZeroThreads = 512;
-constexpr int kZeroLanes = kZeroThreads / kZeroRows;  // threads per row
+constexpr int kZeroThreads = 256;
+constexpr int kZeroSlice = 52 * 1024;
 
-__global__ void __launch_bounds__(kZeroThreads) k_subtract_zero(float* __restrict__ fb, long long chan_stride,
-                                                                long long row0, unsigned row_mask, int nchan,
-                                                                long long nrows) {
-  extern __shared__ float z_smem[];  // [nchan][8]
-  __shared__ double red[2][kZeroThreads / 32][kZeroRows];
-  const int rl = threadIdx.x % kZeroRows, cl = threadIdx.x / kZeroRows;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const long long t = (long long)blockIdx.x * kZeroRows + rl;
-  const bool live = t < nrows;
-  float* x = fb + ((unsigned long long)(row0 + (live ? t : 0)) & (unsigned long long)row_mask);
-  for (int c = cl; c < nchan; c += kZeroLanes) {
-    const unsigned d = (unsigned)__cvta_generic_to_shared(z_smem + c * kZeroRows + rl);
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(d), "l"(x + (long long)c * chan_stride),
-                 "r"(live ? 4 : 0));
+template <bool VEC>
+__global__ void __launch_bounds__(kZeroThreads, 1024 / kZeroThreads)
+    k_subtract_zero(float* __restrict__ fb, long long chan_stride, long long row0, unsigned row_mask, int nchan,
+                    long long nrows, int per) {
+  extern __shared__ float4 z_smem[];  // [per][2]: rows 0..3 and 4..7 of a channel
+  constexpr int kWarps = kZeroThreads / 32;
+  __shared__ double red[kWarps][2][kZeroRows];
+  __shared__ double part[3][2][kZeroRows];  // this slice's sums: read by the whole cluster
+  __shared__ double row_ave[kZeroRows];
+  __shared__ float row_hi[kZeroRows], row_lo[kZeroRows], row_m[kZeroRows];
+  cg::cluster_group cluster = cg::this_cluster();
+  const int nslice = (int)cluster.num_blocks();
+  const int c0 = (int)cluster.block_rank() * per;
+  const int nq = 2 * max(0, min(per, nchan - c0));  // quads of this slice
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, h = tid & 1;
+  const long long t0 = (long long)(blockIdx.x / nslice) * kZeroRows + 4 * h;
+  const int live = (int)max(0LL, min(4LL, nrows - t0));
+  auto row_at = [&](int i) {
+    return (unsigned long long)(row0 + (i < live ? t0 + i : 0)) & (unsigned long long)row_mask;
+  };
+  float* x[VEC ? 1 : 4];
+#pragma unroll
+  for (int i = 0; i < (VEC ? 1 : 4); ++i) x[i] = fb + (c0 + tid / 2) * chan_stride + row_at(i);
+  const long long step = (kZeroThreads / 2) * chan_stride;
+  {
+    long long o = 0;
+    for (int q = tid; q < nq; q += kZeroThreads, o += step) {
+      const unsigned d = (unsigned)__cvta_generic_to_shared(z_smem + q);
+      if constexpr (VEC) {
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(d), "l"(x[0] + o), "r"(4 * live));
+      } else {
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(d + 4 * i), "l"(x[i] + o),
+                       "r"(i < live ? 4 : 0));
+      }
+    }
   }
   asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;\n" ::: "memory");
   // (a thread reads back only what it copied: no barrier needed)
-  auto row_sum2 = [&](double a, double b, double& sa, double& sb) {
-    a += __shfl_xor_sync(0xffffffffu, a, 8);
-    b += __shfl_xor_sync(0xffffffffu, b, 8);
-    a += __shfl_xor_sync(0xffffffffu, a, 16);
-    b += __shfl_xor_sync(0xffffffffu, b, 16);
-    __syncthreads();
-    if (lane < kZeroRows) {
-      red[0][warp][lane] = a;
-      red[1][warp][lane] = b;
-    }
-    __syncthreads();
-    sa = sb = 0.0;
+  // done(row, A, B) with the cluster's sums of a and b over the channels: by one
+  // thread per row (FP64 divisions are dozens of instructions)
+  auto row_sums = [&](int phase, double (&a)[4], double (&b)[4], auto done) {
+    // half of the values are handed over in each step, so a lane ends with one
+    auto fold = [&](bool up, double keep, double other, int o) {
+      return (up ? other : keep) + __shfl_xor_sync(0xffffffffu, up ? keep : other, o);
+    };
+    const bool u16 = lane & 16, u8 = lane & 8, u4 = lane & 4;
+    double v[4];
 #pragma unroll
-    for (int w = 0; w < kZeroThreads / 32; ++w) {
-      sa += red[0][w][rl];
-      sb += red[1][w][rl];
+    for (int i = 0; i < 4; ++i) v[i] = fold(u16, a[i], b[i], 16);
+    v[0] = fold(u8, v[0], v[2], 8);
+    v[1] = fold(u8, v[1], v[3], 8);
+    v[0] = fold(u4, v[0], v[1], 4);
+    v[0] += __shfl_xor_sync(0xffffffffu, v[0], 2);
+    if (!(lane & 2)) red[warp][u16][4 * h + 2 * u8 + u4] = v[0];
+    __syncthreads();
+    if (tid < 2 * kZeroRows) {
+      double v = 0.0;
+#pragma unroll
+      for (int w = 0; w < kWarps; ++w) v += red[w][tid / kZeroRows][tid % kZeroRows];
+      part[phase][tid / kZeroRows][tid % kZeroRows] = v;
     }
+    cluster.sync();
+    if (tid < 2 * kZeroRows) {
+      double v = 0.0;
+      for (int r = 0; r < nslice; ++r)
+        v += cluster.map_shared_rank(&part[phase][tid / kZeroRows][tid % kZeroRows], r)[0];
+      const double w = __shfl_down_sync((1u << 2 * kZeroRows) - 1, v, kZeroRows);
+      if (tid < kZeroRows) done(tid, v, w);
+    }
+    __syncthreads();
   };
-  double s = 0.0, dummy;
-#pragma unroll 4
-  for (int c = cl; c < nchan; c += kZeroLanes) s += (double)z_smem[c * kZeroRows + rl];
-  double tot;
-  row_sum2(s, 0.0, tot, dummy);
-  const double ave = tot / (double)nchan;
-  double d1 = 0.0, d2 = 0.0;
-#pragma unroll 4
-  for (int c = cl; c < nchan; c += kZeroLanes) {
-    const double d = (double)z_smem[c * kZeroRows + rl] - ave;
-    d1 += d;
-    d2 += d * d;
-  }
-  double s1, s2;
-  row_sum2(d1, d2, s1, s2);
   const double n = (double)nchan;
-  const double sig = (s2 - s1 * s1 / n) / (n - 1.0);
-  const float hi = clip_hi(ave + 3.0 * sig), lo = clip_lo(ave - 3.0 * sig);
-  int out = 0;  // values that the clip rejects
-#pragma unroll 4
-  for (int c = cl; c < nchan; c += kZeroLanes) {
-    const float v = z_smem[c * kZeroRows + rl];
-    out += (v < hi && v > lo) ? 0 : 1;
+  double a[4] = {}, b[4] = {};
+#pragma unroll 2
+  for (int q = tid; q < nq; q += kZeroThreads) {
+    const float4 v = z_smem[q];
+    a[0] += (double)v.x;
+    a[1] += (double)v.y;
+    a[2] += (double)v.z;
+    a[3] += (double)v.w;
   }
-  double cs = 0.0, cnt = n;
-  if (__syncthreads_or(out)) {  // some row loses values: sum what is kept
-    int kept = 0;
-    for (int c = cl; c < nchan; c += kZeroLanes) {
-      const float v = z_smem[c * kZeroRows + rl];
-      if (v < hi && v > lo) {
-        cs += (double)v;
-        ++kept;
+  row_sums(0, a, b, [&](int r, double s, double) { row_ave[r] = s / n; });
+  double ave[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    ave[i] = row_ave[4 * h + i];
+    a[i] = b[i] = 0.0;
+  }
+#pragma unroll 2
+  for (int q = tid; q < nq; q += kZeroThreads) {
+    const float4 v = z_smem[q];
+    const float f[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const double d = (double)f[i] - ave[i];
+      a[i] += d;
+      b[i] = fma(d, d, b[i]);
+    }
+  }
+  row_sums(1, a, b, [&](int r, double s1, double s2) {
+    const double sig = (s2 - s1 * s1 / n) / (n - 1.0);
+    row_hi[r] = clip_hi(row_ave[r] + 3.0 * sig);
+    row_lo[r] = clip_lo(row_ave[r] - 3.0 * sig);
+  });
+  float hi[4], lo[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    hi[i] = row_hi[4 * h + i];
+    lo[i] = row_lo[4 * h + i];
+  }
+  bool out = false;  // the clip rejects values of a row
+#pragma unroll 2
+  for (int q = tid; q < nq; q += kZeroThreads) {
+    const float4 v = z_smem[q];
+    const float f[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) out |= i < live && !(f[i] < hi[i] && f[i] > lo[i]);
+  }
+  if (__syncthreads_or(out)) {
+    int kept[4] = {};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) a[i] = 0.0;
+    for (int q = tid; q < nq; q += kZeroThreads) {
+      const float4 v = z_smem[q];
+      const float f[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        if (f[i] < hi[i] && f[i] > lo[i]) {
+          a[i] += (double)f[i];
+          ++kept[i];
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) b[i] = (double)kept[i];
+  } else {  // the slice loses nothing: its sum is the first pass's
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      a[i] = tid < 2 ? part[0][0][4 * h + i] : 0.0;
+      b[i] = tid < 2 ? (double)(nq / 2) : 0.0;
+    }
+  }
+  row_sums(2, a, b, [&](int r, double s, double cnt) { row_m[r] = (float)(s / (cnt > 0.0 ? cnt : 1.0)); });
+  cluster.barrier_arrive();  // this CTA has read the others' sums
+  float m[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) m[i] = row_m[4 * h + i];
+  {
+    long long o = 0;
+#pragma unroll 2
+    for (int q = tid; q < nq; q += kZeroThreads, o += step) {
+      const float4 v = z_smem[q];
+      const float4 y = make_float4(v.x - m[0], v.y - m[1], v.z - m[2], v.w - m[3]);
+      if (VEC && live == 4) {
+        *reinterpret_cast<float4*>(x[0] + o) = y;
+      } else {
+        const float f[4] = {y.x, y.y, y.z, y.w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          if (i < live) (VEC ? x[0] + i : x[VEC ? 0 : i])[o] = f[i];
       }
     }
-    double csum;
-    row_sum2(cs, (double)kept, csum, cnt);
-    cs = csum;
-  } else {
-    cs = tot;
   }
-  const float m = (float)(cs / (cnt > 0.0 ? cnt : 1.0));
-  if (live) {
-#pragma unroll 4
-    for (int c = cl; c < nchan; c += kZeroLanes) x[(long long)c * chan_stride] = z_smem[c * kZeroRows + rl] - m;
-  }
+  cluster.barrier_wait();  // no CTA leaves while another may read its sums
 }
 
 // More channels than fit in shared memory: one thread per row; a warp covers 32
@@ -288,12 +384,33 @@ int launch_subtract_bp_full(float* fb, long long chan_stride, long long row0, un
 int launch_subtract_zero(float* fb, long long chan_stride, long long row0, unsigned row_mask, int nchan,
                          long long nrows, cudaStream_t s) {
   if (!rfi_args_ok(fb, chan_stride, row0, row_mask, nchan, nrows)) return VFRB_ERR_ARG;
-  const long long smem = (long long)nchan * kZeroRows * 4;
+  auto slice = [&](int k) { return (long long)((nchan + k - 1) / k) * kZeroRows * 4; };
+  int k = 1;
+  while (k < 8 && slice(k) > kZeroSlice) k *= 2;
+  const long long smem = slice(k);
   if (smem <= kRfiSmem) {
-    const long long nb = (nrows + kZeroRows - 1) / kZeroRows;
+    const long long nb = (nrows + kZeroRows - 1) / kZeroRows * k;
     if (nb > 0x7fffffffLL) return VFRB_ERR_UNSUPPORTED;
-    if (const int st = rfi_smem(k_subtract_zero)) return st;
-    k_subtract_zero<<<(unsigned)nb, kZeroThreads, (size_t)smem, s>>>(fb, chan_stride, row0, row_mask, nchan, nrows);
+    const bool vec = ((uintptr_t)fb & 15) == 0 && (chan_stride & 3) == 0 && (row0 & 3) == 0 && (row_mask & 3) == 3;
+    auto* kern = vec ? k_subtract_zero<true> : k_subtract_zero<false>;
+    if (const int st = rfi_smem(kern)) return st;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)nb);
+    cfg.blockDim = dim3(kZeroThreads);
+    cfg.dynamicSmemBytes = (size_t)smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at = {};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = (unsigned)k;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, fb, chan_stride, row0, row_mask, nchan, nrows,
+                                             (nchan + k - 1) / k);
+    if (e != cudaSuccess) {
+      cudaGetLastError();
+      return cuda_status(e);
+    }
   } else {
     const long long nb = (nrows + 255) / 256;
     if (nb > 0x7fffffffLL) return VFRB_ERR_UNSUPPORTED;
