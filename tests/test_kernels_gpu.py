@@ -737,3 +737,26 @@ def test_subtract_zero_slices(vf, O, nch, rows, row0, ring):
     assert np.max(np.abs(got[:, idx].T - ref)) <= 1e-6 * np.abs(x).max()
     rest = np.setdiff1d(np.arange(ring), idx)
     assert (got[:, rest] == 7.0).all()
+
+
+@pytest.mark.parametrize("rows,row0,stride", [(3, 0, 64), (2048, 4, 4096), (2049, 4, 4096), (2051, 4095, 4096),
+                                              (8192, 0, 8192), (8190, 8188, 8192), (8193, 0, 8200), (8192, 2, 8196)])
+def test_subtract_bp_full_lengths(vf, O, rows, row0, stride):
+    """Whole-block subtractbp at the lengths where the kernel keeps rows in
+    registers or in shared memory, aligned and unaligned, in a linear run and
+    across a ring's end, within one float rounding of the FP64 oracle; other
+    rows stay as they are."""
+    torch = _torch()
+    x = _rfi_fb(rows, 11, seed=rows)
+    ring = stride & (stride - 1) == 0
+    idx = (row0 + np.arange(rows)) % stride if ring else row0 + np.arange(rows)
+    buf = np.full((11, stride), 7.0, np.float32)
+    buf[:, idx] = x.T
+    cm = torch.from_numpy(buf).cuda()
+    kw = dict(row_mask=stride - 1) if ring else {}
+    vf.subtract_bp_full(cm, nrows=rows, row0=row0, **kw)
+    got, ref = cm.cpu().numpy(), O.subtract_bp_full(x.astype(np.float64))
+    g, ok = got[:, idx].T, ~np.isnan(ref)
+    assert np.array_equal(np.isnan(g), ~ok) and np.max(np.abs(g[ok] - ref[ok])) <= 1e-6 * np.abs(x).max()
+    rest = np.setdiff1d(np.arange(stride), idx)
+    assert (got[:, rest] == 7.0).all()

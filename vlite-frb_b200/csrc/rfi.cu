@@ -14,9 +14,9 @@
 //
 // Sums are FP64 (the reference sums sequentially in FP32).  The statistics need
 // three passes over the same values (mean, variance, clipped mean) and a fourth
-// to subtract.  Both kernels keep the values in shared memory meanwhile, so
-// memory is read once and written once; lengths that do not fit there go
-// through memory four times.
+// to subtract.  Both kernels keep the values in registers or shared memory
+// meanwhile, so memory is read once and written once; lengths that do not fit
+// there go through memory four times.
 #include "vfrb_common.cuh"
 
 #include <cooperative_groups.h>
@@ -41,14 +41,23 @@ __device__ __forceinline__ float clip_hi(double hi) { return __double2float_ru(h
 __device__ __forceinline__ float clip_lo(double lo) { return __double2float_rd(lo); }
 
 // ---- whole-block clipped channel mean ------------------------------------------
-// one CTA (256 threads) per channel.  CACHED: the channel's rows in shared memory
-// (30 kB at 7680 rows: several CTAs per SM hide each other's passes).  7680 rows x
-// 6250 channels: 144 us with four passes over memory, 102 us.
-template <bool CACHED>
-__global__ void __launch_bounds__(256) k_subtract_bp_full(float* __restrict__ fb, long long chan_stride, long long row0,
+// One CTA (256 threads) per channel.  NV > 0: a thread keeps NV rows of the channel
+// in registers, all of their loads in flight at once, in quads of neighbouring rows
+// where these are aligned (VEC).  NV = 0: longer channels, in shared memory (CACHED)
+// or read in every pass.
+//
+// NV = 32 leaves 64 registers a thread, four CTAs per SM; 8192 rows are its limit, and
+// 2048 that of NV = 8, whose loops are short enough for a few hundred rows.  Bound by
+// the FP64 sums and conversions (three per value) and the three reductions.  7680
+// rows x 6250 channels: 144 us with four passes over memory, 102 us through shared
+// memory with 4-byte accesses and every thread dividing, 93 us.
+template <int NV, bool VEC, bool CACHED>
+__global__ void __launch_bounds__(256, NV ? 4 : 1) k_subtract_bp_full(float* __restrict__ fb, long long chan_stride, long long row0,
                                                           unsigned row_mask, int nchan, long long nrows) {
   extern __shared__ float bp_smem[];
-  __shared__ double red[2][8];
+  __shared__ double red[3][2][8];
+  __shared__ double s_ave;
+  __shared__ float s_hi, s_lo, s_m;
   const int c = blockIdx.x;
   float* x = fb + (long long)c * chan_stride;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -56,74 +65,93 @@ __global__ void __launch_bounds__(256) k_subtract_bp_full(float* __restrict__ fb
   const unsigned r0 = (unsigned)row0;
   auto mem = [&](unsigned t) -> float& { return x[(r0 + t) & row_mask]; };
   const unsigned n32 = (unsigned)nrows;
-  auto block_sum2 = [&](double a, double b, double& sa, double& sb) {
+  // done(A, B), by thread 0 (FP64 divisions are dozens of instructions), with the
+  // CTA's sums of a and b
+  auto block_sum2 = [&](int phase, double a, double b, auto done) {
     a = rfi_wsum(a);
     b = rfi_wsum(b);
-    __syncthreads();
     if (lane == 0) {
-      red[0][warp] = a;
-      red[1][warp] = b;
+      red[phase][0][warp] = a;
+      red[phase][1][warp] = b;
     }
     __syncthreads();
-    sa = sb = 0.0;
+    if (threadIdx.x < 16) {
+      double v = red[phase][threadIdx.x >> 3][threadIdx.x & 7];
 #pragma unroll
-    for (int w = 0; w < 8; ++w) {
-      sa += red[0][w];
-      sb += red[1][w];
+      for (int o = 4; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffu, v, o);
+      const double w = __shfl_down_sync(0xffffu, v, 8);
+      if (threadIdx.x == 0) done(v, w);
+    }
+    __syncthreads();
+  };
+  // row of register k; a pass over all rows
+  auto row = [&](int k) { return VEC ? 4 * (threadIdx.x + 256 * (k / 4)) + k % 4 : threadIdx.x + 256 * k; };
+  float v[NV ? NV : 1];
+  if constexpr (NV > 0 && VEC) {
+#pragma unroll
+    for (int k = 0; k < NV; k += 4)
+      if (row(k) < n32) {
+        const float4 q = *reinterpret_cast<const float4*>(&mem(row(k)));
+        v[k] = q.x, v[k + 1] = q.y, v[k + 2] = q.z, v[k + 3] = q.w;
+      }
+  } else if constexpr (NV > 0) {
+#pragma unroll
+    for (int k = 0; k < NV; ++k)
+      if (row(k) < n32) v[k] = mem(row(k));
+  } else if constexpr (CACHED) {  // (a thread reads back only its own rows)
+#pragma unroll 8
+    for (unsigned t = threadIdx.x; t < n32; t += 256) bp_smem[t] = mem(t);
+  }
+  auto each = [&](auto f) {
+    if constexpr (NV > 0) {
+#pragma unroll
+      for (int k = 0; k < NV; ++k)
+        if (row(k) < n32) f(v[k]);
+    } else {
+#pragma unroll 4
+      for (unsigned t = threadIdx.x; t < n32; t += 256) f(CACHED ? bp_smem[t] : mem(t));
     }
   };
-  auto at = [&](unsigned t) -> float { return CACHED ? bp_smem[t] : mem(t); };
-  double s = 0.0, dummy;
-  if (CACHED) {
-    unsigned t = threadIdx.x;
-    for (; t + 7 * 256 < n32; t += 8 * 256) {
-      float v[8];
-#pragma unroll
-      for (int u = 0; u < 8; ++u) v[u] = mem(t + 256 * u);
-#pragma unroll
-      for (int u = 0; u < 8; ++u) {
-        bp_smem[t + 256 * u] = v[u];
-        s += (double)v[u];
-      }
-    }
-    for (; t < n32; t += 256) {
-      const float v = mem(t);
-      bp_smem[t] = v;
-      s += (double)v;
-    }
-  } else {
-    for (unsigned t = threadIdx.x; t < n32; t += 256) s += (double)mem(t);
-  }
-  double tot;
-  block_sum2(s, 0.0, tot, dummy);
-  const double ave = tot / (double)nchan;  // the reference divides by NCHANOUT
+  const double n = (double)nrows;
+  double s = 0.0;
+  each([&](float u) { s += (double)u; });
+  block_sum2(0, s, 0.0, [&](double a, double) { s_ave = a / (double)nchan; });  // the reference divides by NCHANOUT
+  const double ave = s_ave;
   double d1 = 0.0, d2 = 0.0;
-#pragma unroll 4
-  for (unsigned t = threadIdx.x; t < n32; t += 256) {
-    const double d = (double)at(t) - ave;
+  each([&](float u) {
+    const double d = (double)u - ave;
     d1 += d;
     d2 += d * d;
-  }
-  double sum, sum2;
-  block_sum2(d1, d2, sum, sum2);
-  const double n = (double)nrows;
-  const double sig = (sum2 - sum * sum / n) / (n - 1.0);
-  const float hi = clip_hi(ave + 3.0 * sig), lo = clip_lo(ave - 3.0 * sig);
+  });
+  block_sum2(1, d1, d2, [&](double sum, double sum2) {
+    const double sig = (sum2 - sum * sum / n) / (n - 1.0);
+    s_hi = clip_hi(ave + 3.0 * sig);
+    s_lo = clip_lo(ave - 3.0 * sig);
+  });
+  const float hi = s_hi, lo = s_lo;
   double cs = 0.0;
   int cn = 0;
-#pragma unroll 4
-  for (unsigned t = threadIdx.x; t < n32; t += 256) {
-    const float v = at(t);
-    if (v < hi && v > lo) {
-      cs += (double)v;
+  each([&](float u) {
+    if (u < hi && u > lo) {
+      cs += (double)u;
       ++cn;
     }
-  }
-  double csum, cnt;
-  block_sum2(cs, (double)cn, csum, cnt);
-  const float m = (float)(csum / cnt);  // cnt == 0 gives NaN, as the reference's ave/=i
+  });
+  block_sum2(2, cs, (double)cn, [&](double a, double b) { s_m = (float)(a / b); });  // no rows kept: NaN, as the reference's ave/=i
+  const float m = s_m;
+  if constexpr (NV > 0 && VEC) {
+#pragma unroll
+    for (int k = 0; k < NV; k += 4)
+      if (row(k) < n32)
+        *reinterpret_cast<float4*>(&mem(row(k))) = make_float4(v[k] - m, v[k + 1] - m, v[k + 2] - m, v[k + 3] - m);
+  } else if constexpr (NV > 0) {
+#pragma unroll
+    for (int k = 0; k < NV; ++k)
+      if (row(k) < n32) mem(row(k)) = v[k] - m;
+  } else {
 #pragma unroll 4
-  for (unsigned t = threadIdx.x; t < n32; t += 256) mem(t) = at(t) - m;
+    for (unsigned t = threadIdx.x; t < n32; t += 256) mem(t) = (CACHED ? bp_smem[t] : mem(t)) - m;
+  }
 }
 
 // ---- zero-DM ----------------------------------------------------------------------
@@ -358,6 +386,11 @@ static bool rfi_args_ok(const float* fb, long long chan_stride, long long row0, 
   return true;
 }
 
+// rows row0 + 4 i .. + 3 are 16 aligned bytes of memory
+static bool rfi_quads(const float* fb, long long chan_stride, long long row0, unsigned row_mask) {
+  return ((uintptr_t)fb & 15) == 0 && (chan_stride & 3) == 0 && (row0 & 3) == 0 && (row_mask & 3) == 3;
+}
+
 constexpr int kRfiSmem = 220 * 1024;  // of the dynamic kind, beside the sums
 
 template <typename K>
@@ -372,11 +405,19 @@ static int rfi_smem(K kern) {  // one limit, whoever launches
 int launch_subtract_bp_full(float* fb, long long chan_stride, long long row0, unsigned row_mask, int nchan,
                             long long nrows, cudaStream_t s) {
   if (!rfi_args_ok(fb, chan_stride, row0, row_mask, nchan, nrows)) return VFRB_ERR_ARG;
-  if (nrows * 4 <= kRfiSmem) {
-    if (const int st = rfi_smem(k_subtract_bp_full<true>)) return st;
-    k_subtract_bp_full<true><<<nchan, 256, (size_t)nrows * 4, s>>>(fb, chan_stride, row0, row_mask, nchan, nrows);
+  const bool vec = rfi_quads(fb, chan_stride, row0, row_mask) && (nrows & 3) == 0;
+  auto run = [&](auto kern, size_t smem) {
+    kern<<<nchan, 256, smem, s>>>(fb, chan_stride, row0, row_mask, nchan, nrows);
+  };
+  if (nrows <= 8 * 256) {
+    vec ? run(k_subtract_bp_full<8, true, false>, 0) : run(k_subtract_bp_full<8, false, false>, 0);
+  } else if (nrows <= 32 * 256) {
+    vec ? run(k_subtract_bp_full<32, true, false>, 0) : run(k_subtract_bp_full<32, false, false>, 0);
+  } else if (nrows * 4 <= kRfiSmem) {
+    if (const int st = rfi_smem(k_subtract_bp_full<0, false, true>)) return st;
+    run(k_subtract_bp_full<0, false, true>, (size_t)nrows * 4);
   } else {
-    k_subtract_bp_full<false><<<nchan, 256, 0, s>>>(fb, chan_stride, row0, row_mask, nchan, nrows);
+    run(k_subtract_bp_full<0, false, false>, 0);
   }
   return cuda_status(cudaGetLastError());
 }
@@ -391,7 +432,7 @@ int launch_subtract_zero(float* fb, long long chan_stride, long long row0, unsig
   if (smem <= kRfiSmem) {
     const long long nb = (nrows + kZeroRows - 1) / kZeroRows * k;
     if (nb > 0x7fffffffLL) return VFRB_ERR_UNSUPPORTED;
-    const bool vec = ((uintptr_t)fb & 15) == 0 && (chan_stride & 3) == 0 && (row0 & 3) == 0 && (row_mask & 3) == 3;
+    const bool vec = rfi_quads(fb, chan_stride, row0, row_mask);
     auto* kern = vec ? k_subtract_zero<true> : k_subtract_zero<false>;
     if (const int st = rfi_smem(kern)) return st;
     cudaLaunchConfig_t cfg = {};
