@@ -7,6 +7,12 @@
 #include <cstdint>
 #include <vector>
 
+#ifdef __CUDACC__
+#define VFRB_HD __host__ __device__ __forceinline__
+#else
+#define VFRB_HD inline
+#endif
+
 namespace vfrb {
 
 constexpr int kBandD = 8;                 // trials per group
@@ -51,6 +57,23 @@ struct BandHost {
   std::vector<unsigned char> rec;  // [chunk][nblocks][split][gper][rec_bytes]
   std::vector<unsigned> shift;     // [group][nchan] eight shifts, 4 bits each; empty when all are staircases
 };
+
+// Rows [lo, lo + n) of a tile row that starts at row a (a multiple of kBandAlign):
+// the valid rows among its lm in whole groups of vec (16 bytes; the first group may
+// begin before row0), and hi, the end of all its valid rows.  Only valid rows are
+// read: a ring need be no longer than these, so a run of more would meet itself, or
+// pass the ring's end twice.  n <= ring rows: the run is one copy, or two where it
+// passes the end once.
+struct BandRows {
+  long long lo, hi;
+  int n;
+};
+VFRB_HD BandRows band_rows(long long a, int lm, long long row0, long long vend, int vec) {
+  const long long first = (row0 > 0 ? row0 : 0) & ~(long long)(vec - 1);
+  const long long lo = a > first ? a : first, end = a + lm < vend ? a + lm : vend;
+  const long long hi = end > lo ? end : lo;
+  return BandRows{lo, hi, (int)((hi & ~(long long)(vec - 1)) - lo)};
+}
 
 inline long long floor_div(long long a, long long b) { return a >= 0 ? a / b : -((-a + b - 1) / b); }
 inline int floor_to(int a, int b) { return (int)floor_div(a, b) * b; }

@@ -39,8 +39,8 @@
 // 0.78 ms at 1024 samples, where a band has fewer CTAs than the device SMs.
 //
 // A chunk of channels is staged by bulk asynchronous copies into one of two
-// shared-memory buffers while the other is summed (zeros and the last few rows
-// beside the valid ones are written by the warps), with the chunk's sorted
+// shared-memory buffers while the other is summed (zeros outside the valid rows and
+// the last few of them are written by the warps), with the chunk's sorted
 // channel lists (one record per group, made when the plan is created: slots by
 // pattern, and the runs).
 #include "dedisp_band.h"
@@ -346,12 +346,13 @@ __global__ void __launch_bounds__(kBandW * 32, 1) k_dedisp_band(const __grid_con
     const int cn = max(0, min(per, nc - cb));
     const T* src0 = fb + (long long)(p.c_lo + k * CH + cb) * p.chan_stride;
     T* dst0 = s_tile + ((long long)b * CH + cb) * LM;
-    // This lane's channel: rows [lo, hi) of its tile row [a, a + LM) are valid; the
-    // whole 16-byte groups among them come in one bulk copy (two where they wrap
-    // the ring), the warp writes zeros and the last few rows beside them.
+    // This lane's channel: the whole 16-byte groups among the valid rows of its tile
+    // row [a, a + LM) come in one bulk copy (two where they wrap the ring), the warp
+    // writes zeros and the last few rows beside them.
     const long long a = ta + bm;
-    const long long lo = max(a, 0LL), hi = max(lo, min(a + LM, vend));
-    const int nrow = lane < cn ? (int)((hi & ~(long long)(VEC - 1)) - lo) : 0;
+    const BandRows rows_of = band_rows(a, LM, row0, vend, VEC);
+    const long long lo = rows_of.lo, hi = rows_of.hi;
+    const int nrow = lane < cn ? rows_of.n : 0;
     const bool part = lane < cn && nrow < LM;
     unsigned todo = __ballot_sync(0xffffffffu, part);
     while (todo) {
