@@ -40,6 +40,13 @@ struct BandDesc {
 // a group's record of a chunk: slot[ch_cap] (tile offset | channel << 18), run[ch_cap] (code | count << 8), nrun
 constexpr int band_rec_bytes(int ch_cap) { return (ch_cap * 6 + 2 + 15) / 16 * 16; }
 
+// Shared memory of a launch: two mbarriers, two buffers of records, of weights and of
+// tile rows; the rows' place also takes the sums of the longest tile at the end.
+inline size_t band_smem(int ch, int lm, int rec_bytes, int elem, bool weighted) {
+  const size_t fixed = 16 + (size_t)2 * kBandW * rec_bytes + (weighted ? (size_t)2 * ((ch + 3) / 4 * 4) * 4 : 0);
+  return fixed + std::max((size_t)2 * ch * lm * elem, (size_t)kBandW * kBandNtMax * 4);
+}
+
 struct BandHost {
   int ndm = 0, nchan = 0, ngroups = 0, nblocks = 0;
   // Groups per CTA.  Its kBandW warps are `split` sets of them: with fewer
@@ -190,7 +197,11 @@ inline bool band_build(BandHost& h, const int32_t* off, int ndm, int nchan) {
         bmin[(size_t)k * nchan + c] = mn;
         span[bi] = std::max(span[bi], mx - mn);
       }
-  int chunk0 = 0, cap = 1;
+  int cap = 1;
+  auto chunks = [&](BandDesc& b, int most) {
+    b.nchunks = (b.nch + most - 1) / most;
+    b.ch = (b.nch + b.nchunks - 1) / b.nchunks;  // even chunks
+  };
   for (int bi = 0; bi < nbands; ++bi) {
     BandDesc& b = t->bands[bi];
     b.lm = (kBandAlign - 1 + span[bi] + kBandNtMax + kBandSmax + 1 + kBandAlign - 1) / kBandAlign * kBandAlign;
@@ -199,13 +210,21 @@ inline bool band_build(BandHost& h, const int32_t* off, int ndm, int nchan) {
     ch = std::min(ch, kBandMaxCh);
     ch = std::min(ch, 32 * kBandW);
     if (ch < 8) return false;  // the block's trials spread too far to share staged rows
-    b.nchunks = (b.nch + ch - 1) / ch;
-    b.ch = (b.nch + b.nchunks - 1) / b.nchunks;  // even chunks
-    b.chunk0 = chunk0;
-    chunk0 += b.nchunks;
+    chunks(b, ch);
     cap = std::max(cap, (b.ch + SP - 1) / SP);
   }
   cap = (cap + 2) & ~1;  // and a slot of padding, read ahead
+  // Every band's records have the room of the largest chunk's: a band of long rows,
+  // whose own chunks are short, may have to take still fewer channels beside them.
+  int chunk0 = 0;
+  for (BandDesc& b : t->bands) {
+    while (band_smem(b.ch, b.lm, band_rec_bytes(cap), 4, false) > (size_t)kBandSmemMax) {
+      if (b.ch <= 4) return false;
+      chunks(b, b.ch - 1);
+    }
+    b.chunk0 = chunk0;
+    chunk0 += b.nchunks;
+  }
   t->ch_cap = cap;
   t->rec_bytes = band_rec_bytes(cap);
   const size_t ngp = (size_t)nb * G;

@@ -581,8 +581,7 @@ static int band_launch_t(const BandTables* t, BandParams& k, long long nt_max, c
     k.rec = t->d_rec + (size_t)b.chunk0 * nb * kBandW * t->h.rec_bytes;
     k.first = bi == 0;
     k.last = bi == nbands - 1;
-    const size_t fixed = 16 + (size_t)2 * kBandW * t->h.rec_bytes + (WT ? (size_t)2 * ((b.ch + 3) / 4 * 4) * 4 : 0);
-    const size_t smem = fixed + std::max((size_t)2 * b.ch * b.lm * sizeof(T), (size_t)kBandW * NT * 4);
+    const size_t smem = band_smem(b.ch, b.lm, t->h.rec_bytes, sizeof(T), WT);
     const dim3 grid((unsigned)nb, gy[bi], (unsigned)std::max(1, k.njobs));
     // A band overlaps the one before it (programmatic dependent launch): its
     // CTAs fill the SMs that the last wave leaves free, and stage and sum their
