@@ -87,25 +87,27 @@ __global__ void __launch_bounds__(kBoxThreads) k_boxcar_tree(const float* __rest
   const float* x = dd + (long long)d * stride;
   const double a = (double)ave[d];
   const double s = (double)sigma[d];
-  const int n = (int)nt;
   BoxBest best{-INFINITY, 0x7fffffff, 0x7fffffff};
-  for (int t0 = 0; t0 < n; t0 += kBoxTile) {
+  // (64-bit tile starts: nt may be the largest int, past which the last step goes)
+  for (long long t0 = 0; t0 < nt; t0 += kBoxTile) {
+    const float* xt = x + t0;
+    const int have = (int)min(nt - t0, (long long)(kBoxTile + kBoxTree));  // samples of the tile that there are
     // this thread's samples: tid + 256 i, the last of them in the halo
     double v[kBoxPer + 1];
 #pragma unroll
     for (int i = 0; i <= kBoxPer; ++i) {
       const int p = tid + kBoxThreads * i;
-      v[i] = p < kBoxTile + wmax - 1 && t0 + p < n ? (double)x[t0 + p] : 0.0;
+      v[i] = p < kBoxTile + wmax - 1 && p < have ? (double)xt[p] : 0.0;
     }
     for (int w = 1;; w *= 2) {
       const double wa = (double)w * a, inv = 1.0 / (s * sqrt((double)w));
-      const int last = n - w - t0;  // starts t0 + p <= nt - w
+      const int last = have - w;  // starts t0 + p <= nt - w
 #pragma unroll
       for (int i = 0; i < kBoxPer; ++i) {
         const int p = tid + kBoxThreads * i;
         const double q = (v[i] - wa) * inv;
         // ties: the smaller width (tiles are walked in time, so the earlier start of a width comes first)
-        if (p <= last && (q > best.snr || (q == best.snr && w < best.w))) best = BoxBest{q, t0 + p, w};
+        if (p <= last && (q > best.snr || (q == best.snr && w < best.w))) best = BoxBest{q, (int)t0 + p, w};
       }
       if (2 * w > wmax) break;
       __syncthreads();  // the half width's (or the last tile's) sums have been read
