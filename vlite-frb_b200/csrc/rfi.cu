@@ -17,6 +17,7 @@
 // to subtract.  Both kernels keep the values in registers or shared memory
 // meanwhile, so memory is read once and written once; lengths that do not fit
 // there go through memory four times.
+#include "rfi_rows.h"
 #include "vfrb_common.cuh"
 
 #include <cooperative_groups.h>
@@ -61,10 +62,11 @@ __global__ void __launch_bounds__(256, NV ? 4 : 1) k_subtract_bp_full(float* __r
   const int c = blockIdx.x;
   float* x = fb + (long long)c * chan_stride;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  // 32-bit row arithmetic is enough: the ring's (or linear run's) rows are below 2^32
+  // rows are taken modulo 2^32, the widest mask; their count may be larger (NV = 0)
   const unsigned r0 = (unsigned)row0;
   auto mem = [&](unsigned t) -> float& { return x[(r0 + t) & row_mask]; };
-  const unsigned n32 = (unsigned)nrows;
+  using Row = BpFullRow<NV == 0 && !CACHED>;
+  const Row n = (Row)nrows;
   // done(A, B), by thread 0 (FP64 divisions are dozens of instructions), with the
   // CTA's sums of a and b
   auto block_sum2 = [&](int phase, double a, double b, auto done) {
@@ -90,29 +92,27 @@ __global__ void __launch_bounds__(256, NV ? 4 : 1) k_subtract_bp_full(float* __r
   if constexpr (NV > 0 && VEC) {
 #pragma unroll
     for (int k = 0; k < NV; k += 4)
-      if (row(k) < n32) {
+      if (row(k) < n) {
         const float4 q = *reinterpret_cast<const float4*>(&mem(row(k)));
         v[k] = q.x, v[k + 1] = q.y, v[k + 2] = q.z, v[k + 3] = q.w;
       }
   } else if constexpr (NV > 0) {
 #pragma unroll
     for (int k = 0; k < NV; ++k)
-      if (row(k) < n32) v[k] = mem(row(k));
+      if (row(k) < n) v[k] = mem(row(k));
   } else if constexpr (CACHED) {  // (a thread reads back only its own rows)
-#pragma unroll 8
-    for (unsigned t = threadIdx.x; t < n32; t += 256) bp_smem[t] = mem(t);
+    bp_full_rows<8, Row>(threadIdx.x, n, [&](Row t) { bp_smem[t] = mem(t); });
   }
   auto each = [&](auto f) {
     if constexpr (NV > 0) {
 #pragma unroll
       for (int k = 0; k < NV; ++k)
-        if (row(k) < n32) f(v[k]);
+        if (row(k) < n) f(v[k]);
     } else {
-#pragma unroll 4
-      for (unsigned t = threadIdx.x; t < n32; t += 256) f(CACHED ? bp_smem[t] : mem(t));
+      bp_full_rows<4, Row>(threadIdx.x, n, [&](Row t) { f(CACHED ? bp_smem[t] : mem((unsigned)t)); });
     }
   };
-  const double n = (double)nrows;
+  const double nd = (double)nrows;
   double s = 0.0;
   each([&](float u) { s += (double)u; });
   block_sum2(0, s, 0.0, [&](double a, double) { s_ave = a / (double)nchan; });  // the reference divides by NCHANOUT
@@ -124,7 +124,7 @@ __global__ void __launch_bounds__(256, NV ? 4 : 1) k_subtract_bp_full(float* __r
     d2 += d * d;
   });
   block_sum2(1, d1, d2, [&](double sum, double sum2) {
-    const double sig = (sum2 - sum * sum / n) / (n - 1.0);
+    const double sig = (sum2 - sum * sum / nd) / (nd - 1.0);
     s_hi = clip_hi(ave + 3.0 * sig);
     s_lo = clip_lo(ave - 3.0 * sig);
   });
@@ -142,15 +142,17 @@ __global__ void __launch_bounds__(256, NV ? 4 : 1) k_subtract_bp_full(float* __r
   if constexpr (NV > 0 && VEC) {
 #pragma unroll
     for (int k = 0; k < NV; k += 4)
-      if (row(k) < n32)
+      if (row(k) < n)
         *reinterpret_cast<float4*>(&mem(row(k))) = make_float4(v[k] - m, v[k + 1] - m, v[k + 2] - m, v[k + 3] - m);
   } else if constexpr (NV > 0) {
 #pragma unroll
     for (int k = 0; k < NV; ++k)
-      if (row(k) < n32) mem(row(k)) = v[k] - m;
+      if (row(k) < n) mem(row(k)) = v[k] - m;
   } else {
-#pragma unroll 4
-    for (unsigned t = threadIdx.x; t < n32; t += 256) mem(t) = (CACHED ? bp_smem[t] : mem(t)) - m;
+    bp_full_rows<4, Row>(threadIdx.x, n, [&](Row t) {
+      float& at = mem((unsigned)t);
+      at = (CACHED ? bp_smem[t] : at) - m;
+    });
   }
 }
 
