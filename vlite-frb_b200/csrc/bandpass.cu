@@ -21,6 +21,7 @@
 // addresses through the rings' masks; where a window does not wrap a ring (all but
 // one in a ring's length) rows are pointer steps.  7680 rows x 6250 channels: 201 ->
 // 92 us; FP16 with the shifted copy, 1024 rows: 37 -> 22 us.
+#include "row_walk.h"
 #include "vfrb_common.cuh"
 
 #include <algorithm>
@@ -276,7 +277,7 @@ __global__ void __launch_bounds__(256) k_chan_stats(const __grid_constant__ vfrb
   const int npts = (int)(colmax - colmin);
   const float* base = a.fb + (long long)c * a.chan_stride;
   const unsigned r0 = (unsigned)(a.row0 + colmin);  // ring rows are 32-bit
-  auto at = [&](int i) { return base[(r0 + (unsigned)i) & a.row_mask]; };
+  auto at = [&](unsigned i) { return base[(r0 + i) & a.row_mask]; };
   // sums over the group's warps, the same on every lane
   auto group_sum = [&](double& u, double& v) {
     u = warp_sum(u);
@@ -302,7 +303,7 @@ __global__ void __launch_bounds__(256) k_chan_stats(const __grid_constant__ vfrb
       for (int i = 0; i < R; ++i)
         if (FULL || gl + 32 * G * i < npts) f(x[i]);
     } else {
-      for (int i = gl; i < npts; i += 32) f(at(i));
+      walk_rows<32, 4, StatsRow>(gl, npts, [&](StatsRow i) { f(at(i)); });
     }
   };
   if constexpr (NW != 0) {

@@ -17,7 +17,7 @@
 // to subtract.  Both kernels keep the values in registers or shared memory
 // meanwhile, so memory is read once and written once; lengths that do not fit
 // there go through memory four times.
-#include "rfi_rows.h"
+#include "row_walk.h"
 #include "vfrb_common.cuh"
 
 #include <cooperative_groups.h>
@@ -101,7 +101,7 @@ __global__ void __launch_bounds__(256, NV ? 4 : 1) k_subtract_bp_full(float* __r
     for (int k = 0; k < NV; ++k)
       if (row(k) < n) v[k] = mem(row(k));
   } else if constexpr (CACHED) {  // (a thread reads back only its own rows)
-    bp_full_rows<8, Row>(threadIdx.x, n, [&](Row t) { bp_smem[t] = mem(t); });
+    walk_rows<kBpFullThreads, 8, Row>(threadIdx.x, n, [&](Row t) { bp_smem[t] = mem(t); });
   }
   auto each = [&](auto f) {
     if constexpr (NV > 0) {
@@ -109,7 +109,7 @@ __global__ void __launch_bounds__(256, NV ? 4 : 1) k_subtract_bp_full(float* __r
       for (int k = 0; k < NV; ++k)
         if (row(k) < n) f(v[k]);
     } else {
-      bp_full_rows<4, Row>(threadIdx.x, n, [&](Row t) { f(CACHED ? bp_smem[t] : mem((unsigned)t)); });
+      walk_rows<kBpFullThreads, 4, Row>(threadIdx.x, n, [&](Row t) { f(CACHED ? bp_smem[t] : mem((unsigned)t)); });
     }
   };
   const double nd = (double)nrows;
@@ -149,7 +149,7 @@ __global__ void __launch_bounds__(256, NV ? 4 : 1) k_subtract_bp_full(float* __r
     for (int k = 0; k < NV; ++k)
       if (row(k) < n) mem(row(k)) = v[k] - m;
   } else {
-    bp_full_rows<4, Row>(threadIdx.x, n, [&](Row t) {
+    walk_rows<kBpFullThreads, 4, Row>(threadIdx.x, n, [&](Row t) {
       float& at = mem((unsigned)t);
       at = (CACHED ? bp_smem[t] : at) - m;
     });
