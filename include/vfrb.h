@@ -195,6 +195,12 @@ int vfrb_ddplan_group_size(const vfrb_ddplan* plan);
 #define VFRB_DD_NVARIANTS 8
 int vfrb_ddplan_set_variant(vfrb_ddplan* plan, int storage, int variant);
 int vfrb_ddplan_variant(const vfrb_ddplan* plan, int storage);
+/* The dedispersion kernels' waits for their own copies are bounded; a call
+ * whose wait gives up ends by itself and adds 8 to its d_err, and its outputs
+ * are not whole.  on != 0: in FP32 calls of the band-wise and the pattern
+ * kernels they give up at once, which is how that path is tested (no reference
+ * counterpart). */
+int vfrb_ddplan_set_give_up(vfrb_ddplan* plan, int on);
 /* Times every applicable variant on scratch data of the given shape
  * (nt_out samples per trial, `storage` form) and keeps the fastest for calls
  * that neither of AUTO's own kernels takes (see VFRB_DD_AUTO).  Writes

@@ -106,6 +106,7 @@ _lib.vfrb_ddplan_max_delay.argtypes = [C.c_void_p]
 _lib.vfrb_ddplan_group_size.argtypes = [C.c_void_p]
 _lib.vfrb_ddplan_set_variant.argtypes = [C.c_void_p, C.c_int, C.c_int]
 _lib.vfrb_ddplan_variant.argtypes = [C.c_void_p, C.c_int]
+_lib.vfrb_ddplan_set_give_up.argtypes = [C.c_void_p, C.c_int]
 _lib.vfrb_ddplan_autotune.argtypes = [C.c_void_p, C.c_int, C.c_int64, C.c_void_p, C.c_void_p]
 _lib.vfrb_dedisperse_workspace_bytes.restype = C.c_size_t
 _lib.vfrb_dedisperse_workspace_bytes.argtypes = [C.c_void_p, C.c_int64]
@@ -257,6 +258,10 @@ class DedispPlan:
 
     def variant(self, storage: int = F32) -> int:
         return int(_lib.vfrb_ddplan_variant(self._p, storage))
+
+    def set_give_up(self, on: bool):
+        """The kernels' bounded waits for their own copies give up at once (vfrb_ddplan_set_give_up)."""
+        _check(_lib.vfrb_ddplan_set_give_up(self._p, int(on)), "vfrb_ddplan_set_give_up")
 
     def autotune(self, storage: int, nt_out: int, stream=None):
         """Times each applicable kernel variant; returns {variant: ms} (n/a omitted)."""

@@ -16,8 +16,9 @@ void band_destroy(BandTables* t);
 // The dedispersed series of one call (njobs == 0) or of the jobs of a batched
 // launch (grid z = job; the fields of `a` that DdJob holds are ignored).
 // *launched = 0 when the call's layout does not suit the kernel: nothing has
-// been launched then.
-int band_launch(const BandTables* t, const vfrb_dd_args& a, const DdJob* jobs, int njobs, cudaStream_t s,
-                int* launched);
+// been launched then.  give_up (FP32): waits for staged rows give up at once, and the
+// call is flagged.
+int band_launch(const BandTables* t, const vfrb_dd_args& a, const DdJob* jobs, int njobs, bool give_up,
+                cudaStream_t s, int* launched);
 
 }  // namespace vfrb

@@ -566,6 +566,7 @@ struct vfrb_ddplan {
   // the others when they have been timed, else the default
   int tuned[3] = {0, 0, 0};
   vfrb::BandTables* band = nullptr;
+  bool give_up = false;             // the kernels' waits for their own copies give up at once
 };
 
 namespace vfrb {
@@ -754,6 +755,7 @@ static int pat_launch_t(const vfrb_ddplan* pl, const RegGroup& g, const vfrb_dd_
   k.chunk = chunk;
   k.lmax = lm;
   k.err = a.d_err;
+  k.give_up = pl->give_up;
   k.njobs = njobs;
   for (int i = 0; i < njobs; ++i) k.jobs[i] = jobs[i];
   const size_t meta = 16 + ((size_t)3 * W * chunk + W + 3) / 4 * 16;
@@ -860,7 +862,7 @@ static int launch_auto(const vfrb_ddplan* pl, const vfrb_dd_args& a, cudaStream_
     else if (a.storage == VFRB_F16) st = few_launch_t<__half, false>(pl, k, s, launched);
     else st = few_launch_t<int8_t, false>(pl, k, s, launched);
   } else if (pl->band && !a.sigma_out) {
-    st = band_launch(pl->band, a, nullptr, 0, s, launched);
+    st = band_launch(pl->band, a, nullptr, 0, pl->give_up, s, launched);
   }
   if (st || !*launched || !want_stats) return st;
   DmPartial* part = reinterpret_cast<DmPartial*>(a.workspace);
@@ -959,7 +961,7 @@ int launch_dedisperse_jobs(const vfrb_ddplan* pl, int storage, const DdJob* jobs
   a.out = jobs[0].out;
   a.out_stride = jobs[0].out_stride;
   if (band) {
-    const int st = band_launch(pl->band, a, jobs, njobs, s, launched);
+    const int st = band_launch(pl->band, a, jobs, njobs, pl->give_up, s, launched);
     if (st || *launched) return st;
     if (v != VFRB_DD_PAT4 && v != VFRB_DD_PAT2) return VFRB_OK;
   }
@@ -1084,6 +1086,12 @@ int ddplan_set_variant(vfrb_ddplan* pl, int storage, int v) {
     if (st) return st;
   }
   pl->variant[storage] = v;
+  return VFRB_OK;
+}
+
+int ddplan_set_give_up(vfrb_ddplan* pl, int on) {
+  if (!pl) return VFRB_ERR_ARG;
+  pl->give_up = on != 0;
   return VFRB_OK;
 }
 

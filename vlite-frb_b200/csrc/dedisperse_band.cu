@@ -281,7 +281,9 @@ struct BandTT<int8_t> {
 // first band's launch is an ordinary one: nothing to wait for).
 __device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
-template <typename T, bool WT>
+// GIVE_UP: waits for staged rows give up at once (a test's form; as a launch parameter it
+// cost 1% of the 201-trial case)
+template <typename T, bool WT, bool GIVE_UP>
 __global__ void __launch_bounds__(kBandW * 32, 1) k_dedisp_band(const __grid_constant__ BandParams p) {
   constexpr int TT = BandTT<T>::v;
   constexpr int NT = 32 * TT;
@@ -314,7 +316,6 @@ __global__ void __launch_bounds__(kBandW * 32, 1) k_dedisp_band(const __grid_con
   const T* fb = reinterpret_cast<const T*>(batch ? job.fb : p.fb);
   const unsigned long long rmask = (unsigned long long)p.row_mask;
   const int CH = p.ch, LM = p.lm;
-  int err = 0;
 
   // shared: full[2] mbarriers | rec[2][W][rec_bytes] | wts[2][CH] (WT) | tile[2][CH][LM]
   extern __shared__ __align__(128) unsigned char band_smem[];
@@ -405,14 +406,17 @@ __global__ void __launch_bounds__(kBandW * 32, 1) k_dedisp_band(const __grid_con
   stage(0, 0, first_rows(0));
   int bm_next = first_rows(1);
   const int lane_off = lane * TT + phase;
-  for (int k = 0; k < nchunks; ++k) {
+  int k = 0;  // nchunks at the end; one more where this warp's wait gave up
+  for (; k < nchunks; ++k) {
     __syncthreads();  // every warp is done with chunk k - 1: its buffer can be refilled
     const int b = k & 1;
     if (k + 1 < nchunks) stage(k + 1, b ^ 1, bm_next);
     bm_next = first_rows(k + 2);
-    if (!mbar_wait(&s_full[b], (unsigned)(k >> 1) & 1u)) {
-      err |= kErrTimeout;
-      continue;  // nothing was staged: the result is flagged
+    if (__any_sync(0xffffffffu, GIVE_UP || !mbar_wait(&s_full[b], (unsigned)(k >> 1) & 1u))) {
+      drain_copies(s_full, k, nchunks);
+      while (++k < nchunks) __syncthreads();  // the other warps' barriers
+      k = nchunks + 1;
+      break;
     }
     const unsigned char* rec = s_rec + ((long long)b * W + warp) * p.rec_bytes;
     const unsigned* slot = reinterpret_cast<const unsigned*>(rec);
@@ -502,7 +506,7 @@ __global__ void __launch_bounds__(kBandW * 32, 1) k_dedisp_band(const __grid_con
     else __syncthreads();
   }
   int* derr = batch ? job.err : p.err;
-  if (err && derr) atomicOr(derr, err);
+  if (k > nchunks && lane == 0 && derr) atomicOr(derr, kErrTimeout);  // the sums are not whole
 }
 
 // ---- host side ------------------------------------------------------------------
@@ -547,7 +551,7 @@ int band_create(BandTables** out, const int32_t* off, int ndm, int nchan) {
   return VFRB_OK;
 }
 
-template <typename T, bool WT>
+template <typename T, bool WT, bool GIVE_UP = false>
 static int band_launch_t(const BandTables* t, BandParams& k, long long nt_max, cudaStream_t s, int* launched) {
   constexpr int NT = 32 * BandTT<T>::v;
   const int nb = t->h.nblocks;
@@ -565,7 +569,7 @@ static int band_launch_t(const BandTables* t, BandParams& k, long long nt_max, c
     gy[bi] = (unsigned)most;
   }
   // one limit for every band and plan: launches of other threads set the same
-  if (cudaFuncSetAttribute(k_dedisp_band<T, WT>, cudaFuncAttributeMaxDynamicSharedMemorySize, kBandSmemMax) !=
+  if (cudaFuncSetAttribute(k_dedisp_band<T, WT, GIVE_UP>, cudaFuncAttributeMaxDynamicSharedMemorySize, kBandSmemMax) !=
       cudaSuccess) {
     cudaGetLastError();
     return VFRB_ERR_CUDA;
@@ -597,7 +601,7 @@ static int band_launch_t(const BandTables* t, BandParams& k, long long nt_max, c
     at.val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = &at;
     cfg.numAttrs = bi > 0 ? 1 : 0;
-    const int st = cuda_status(cudaLaunchKernelEx(&cfg, k_dedisp_band<T, WT>, k));
+    const int st = cuda_status(cudaLaunchKernelEx(&cfg, k_dedisp_band<T, WT, GIVE_UP>, k));
     if (st) {
       cudaGetLastError();
       return st;
@@ -607,8 +611,8 @@ static int band_launch_t(const BandTables* t, BandParams& k, long long nt_max, c
   return VFRB_OK;
 }
 
-int band_launch(const BandTables* t, const vfrb_dd_args& a, const DdJob* jobs, int njobs, cudaStream_t s,
-                int* launched) {
+int band_launch(const BandTables* t, const vfrb_dd_args& a, const DdJob* jobs, int njobs, bool give_up,
+                cudaStream_t s, int* launched) {
   *launched = 0;
   if (!t) return VFRB_OK;
   const int vec = a.storage == VFRB_F32 ? 4 : a.storage == VFRB_F16 ? 8 : 16;
@@ -642,7 +646,9 @@ int band_launch(const BandTables* t, const vfrb_dd_args& a, const DdJob* jobs, i
   k.ch_cap = t->h.ch_cap;
   k.err = a.d_err;
   switch (a.storage) {
-    case VFRB_F32: return band_launch_t<float, false>(t, k, nt, s, launched);
+    case VFRB_F32:
+      return give_up ? band_launch_t<float, false, true>(t, k, nt, s, launched)
+                     : band_launch_t<float, false>(t, k, nt, s, launched);
     case VFRB_F16:
       return weighted ? band_launch_t<__half, true>(t, k, nt, s, launched)
                       : band_launch_t<__half, false>(t, k, nt, s, launched);

@@ -65,6 +65,7 @@ struct DdPatParams {
   int chunk;                   // channels per stage (<= 32)
   int lmax;                    // tile row length in elements (multiple of 16 bytes)
   int* err;
+  int give_up;                 // waits for staged rows give up at once
 };
 
 template <typename T>
@@ -522,7 +523,12 @@ __global__ void __launch_bounds__(W * 32, 16 / W) k_dedisp_pat(const DdPatParams
     sb_next = stage_bmin(k + 2);
     meta(k, m_cur);
     m_cur = meta_in(k + 1);
-    if (!mbar_wait(&s_full[k & 1], (unsigned)(k >> 1) & 1u)) err |= kErrTimeout;
+    if (__any_sync(0xffffffffu, pp.give_up || !mbar_wait(&s_full[k & 1], (unsigned)(k >> 1) & 1u))) {
+      err |= kErrTimeout;  // the sums are not whole
+      drain_copies(s_full, k, nchunks);
+      while (++k < nchunks) __syncthreads();  // the other warps' barriers
+      break;
+    }
     const int b = k & 1;
     const T* tile = reinterpret_cast<const T*>(tiles + (long long)b * NCOPY * CH * LMQ);
     const int mb = warp * CH;
