@@ -464,7 +464,12 @@ int64_t vfrb_plan_device_bytes(const vfrb_plan* plan);
  * pair reader.  Device input is read after all work queued before the call
  * on the legacy default stream (PyTorch's default stream); input written on
  * another stream must be complete (that stream synchronised) before the
- * call.  `bytes` may be reused as soon as the call returns. */
+ * call.  `bytes` may be reused as soon as the call returns.
+ * Pageable host memory goes through two staging buffers: 16 frames each from
+ * the stream's opening, and page-locked for longer runs (up to 41 MB each) in
+ * the first two pushes that bring one -- some ms each, once; where that fails
+ * the small ones serve on, in smaller copies.  Page-locked and device memory
+ * need none of them. */
 int vfrb_push_frames(vfrb_plan* plan, int stream, const uint8_t* bytes, size_t nbytes);
 
 /* Streams opened and closed while others run (serving).  vfrb_stream_open

@@ -30,6 +30,7 @@
 
 #include <nvtx3/nvToolsExt.h>
 
+#include "stage_buffer.h"
 #include "vdif_reader.h"
 #include "vfrb_common.cuh"
 
@@ -77,6 +78,7 @@ constexpr int kStash = 1024;       // gap-revealing frames kept aside per stream
 constexpr int kMaxStreams = 4096;  // stream ids over a plan's life
 constexpr int kSlotBufs = 32;  // rotating slot-table uploads in flight (host runs ahead of the GPU)
 constexpr int kStageBufs = 2;  // rotating staging buffers for pageable input
+constexpr size_t kStageFew = 16;  // frames each holds from the stream's opening on
 
 static unsigned long long pow2_at_least(unsigned long long v) {
   unsigned long long r = 1;
@@ -181,8 +183,7 @@ struct StreamSt {
   int64_t ring_frames = 0;
   int64_t frames_in = 0;       // frames received (ring position)
   int stash_next = 0;
-  uint8_t* h_stage[kStageBufs] = {};
-  size_t stage_cap[kStageBufs] = {};  // frames each holds (made when first needed)
+  StageBuffer stage[kStageBufs];
   // device input: each batch's 32-byte frame headers, packed in
   // page-locked host memory by one strided copy
   uint8_t* h_hdr = nullptr;
@@ -995,17 +996,6 @@ int64_t oldest_ref(const StreamSt* s) {
   return o;
 }
 
-// Staging buffer k holds at least nb frames.  A frame that straddles pushes comes
-// alone: a small buffer for those, the whole one when a longer run comes.  (The
-// buffer it replaces stays with the stream: copies from it may be in flight.)
-int stage_buffer(StreamSt* s, int k, size_t nb) {
-  if (s->stage_cap[k] >= nb) return VFRB_OK;
-  const size_t cap = nb <= 16 ? 16 : s->stage_frames;
-  ST(hmalloc(s->res, &s->h_stage[k], std::max(cap, nb) * kFrameLen));
-  s->stage_cap[k] = std::max(cap, nb);
-  return VFRB_OK;
-}
-
 // Copy `nf` whole frames to the ring, queue their headers, advance.
 int feed_frames(vfrb_plan* pl, StreamSt* s, const uint8_t* in, int64_t nf, MemKind kind) {
   const Range nvtx_range("vfrb feed frames");
@@ -1017,7 +1007,15 @@ int feed_frames(vfrb_plan* pl, StreamSt* s, const uint8_t* in, int64_t nf, MemKi
       1, pinned || device ? s->ring_frames / 4 : std::min<int64_t>(s->ring_frames / 4, (int64_t)s->stage_frames));
   size_t pitch = kFrameLen;  // of the headers the reader reads
   for (int64_t done = 0; done < nf;) {
-    const int64_t nb = std::min(batch_max, nf - done);
+    int64_t nb = std::min(batch_max, nf - done);
+    // page-locking the staging buffers (up to 41 MB each) was most of a stream's
+    // opening: they hold kStageFew frames then (a frame that straddles pushes comes
+    // alone), and grow when pageable input first brings more
+    if (!pinned && !device)
+      nb = (int64_t)stage_room(s->stage[s->stage_i], (size_t)nb, s->stage_frames, [&](size_t frames) {
+        uint8_t* q = nullptr;
+        return hmalloc(s->res, &q, frames * kFrameLen) == VFRB_OK ? q : nullptr;
+      });
     const uint8_t* src = in + done * kFrameLen;  // host bytes, or device bytes (device input)
     // frames about to be overwritten must have been consumed by launched work
     if (oldest_ref(s) < s->frames_in + nb - s->ring_frames) {
@@ -1063,11 +1061,8 @@ int feed_frames(vfrb_plan* pl, StreamSt* s, const uint8_t* in, int64_t nf, MemKi
       const int k = s->stage_i;
       s->stage_i = (s->stage_i + 1) % kStageBufs;
       CK(cudaEventSynchronize(s->stage_ev[k]));
-      // page-locking these (up to 41 MB each) is most of a stream's opening: they
-      // are made when pageable input first needs one of its size
-      ST(stage_buffer(s, k, (size_t)nb));
-      std::memcpy(s->h_stage[k], src, (size_t)nb * kFrameLen);
-      from = s->h_stage[k];
+      std::memcpy(s->stage[k].p, src, (size_t)nb * kFrameLen);
+      from = s->stage[k].p;
       // the staging event is recorded after the copies below
       const int64_t slot0 = s->frames_in % s->ring_frames;
       const int64_t n1 = std::min(nb, s->ring_frames - slot0);
@@ -1151,6 +1146,8 @@ int create_stream(vfrb_plan* pl, int id, int64_t ring_frames, int64_t R1, int64_
   s->stage_frames = (size_t)std::min<int64_t>(ring_frames / 4, 8192);
   ST(hmalloc(s->res, &s->h_hdr, (size_t)std::max<int64_t>(1, ring_frames / 4) * kHdrLen));
   for (int k = 0; k < kStageBufs; ++k) {
+    s->stage[k].frames = std::min(kStageFew, s->stage_frames);
+    ST(hmalloc(s->res, &s->stage[k].p, s->stage[k].frames * kFrameLen));
     ST(mkevent(s->res, &s->stage_ev[k]));
     CK(cudaEventRecord(s->stage_ev[k], s->xs));
   }
