@@ -847,6 +847,10 @@ static DdKParams dd_params(const vfrb_ddplan* pl, const vfrb_dd_args& a) {
   return k;
 }
 
+// samples of a part: 32768 of the streaming kernel's blocks, 16384 band tiles (int8),
+// beside which a band's delays may take the other 49,000 tiles, 12.6 million rows
+constexpr long long kAutoPart = 1LL << 22;
+
 // AUTO's own kernels -- streaming for few trials, band-wise for more -- with the
 // statistics from the finished series; *launched = 0 when neither applies.
 static int launch_auto(const vfrb_ddplan* pl, const vfrb_dd_args& a, cudaStream_t s, int* launched) {
@@ -854,17 +858,30 @@ static int launch_auto(const vfrb_ddplan* pl, const vfrb_dd_args& a, cudaStream_
   const bool want_stats = a.ave || a.sigma || a.peak || a.frb || a.argmax;
   const long long ntb = (a.nt_out + kPartNt - 1) / kPartNt;
   if (want_stats && ntb * pl->ndm > 0x7fffffffLL) return VFRB_OK;
-  int st = VFRB_OK;
-  if (pl->ndm <= (a.sigma_out ? kFewTrialsSigma : kFewTrials)) {
-    const DdKParams k = dd_params(pl, a);
-    if (a.sigma_out) st = few_launch_t<float, true>(pl, k, s, launched);
-    else if (a.storage == VFRB_F32) st = few_launch_t<float, false>(pl, k, s, launched);
-    else if (a.storage == VFRB_F16) st = few_launch_t<__half, false>(pl, k, s, launched);
-    else st = few_launch_t<int8_t, false>(pl, k, s, launched);
-  } else if (pl->band && !a.sigma_out) {
-    st = band_launch(pl->band, a, nullptr, 0, pl->give_up, s, launched);
+  // The kernels' time blocks are a grid's second dimension, of 65535 at most: longer
+  // calls run in parts (a sample's sums do not depend on the cut).
+  for (long long t0 = 0; t0 < a.nt_out; t0 += kAutoPart) {
+    vfrb_dd_args b = a;
+    b.row0 += t0;
+    b.nrows_valid -= t0;
+    b.nt_out = std::min(a.nt_out - t0, kAutoPart);
+    b.out += t0;
+    if (b.sigma_out) b.sigma_out += t0;
+    int st = VFRB_OK, part = 0;
+    if (pl->ndm <= (a.sigma_out ? kFewTrialsSigma : kFewTrials)) {
+      const DdKParams k = dd_params(pl, b);
+      if (a.sigma_out) st = few_launch_t<float, true>(pl, k, s, &part);
+      else if (a.storage == VFRB_F32) st = few_launch_t<float, false>(pl, k, s, &part);
+      else if (a.storage == VFRB_F16) st = few_launch_t<__half, false>(pl, k, s, &part);
+      else st = few_launch_t<int8_t, false>(pl, k, s, &part);
+    } else if (pl->band && !a.sigma_out) {
+      st = band_launch(pl->band, b, nullptr, 0, pl->give_up, s, &part);
+    }
+    if (st) return st;
+    if (!part) return VFRB_OK;  // (of every part or of none: it is the list or the layout that does not suit)
   }
-  if (st || !*launched || !want_stats) return st;
+  *launched = 1;
+  if (!want_stats) return VFRB_OK;
   DmPartial* part = reinterpret_cast<DmPartial*>(a.workspace);
   k_series_part<<<(unsigned)(ntb * pl->ndm), 256, 0, s>>>(a.out, a.nt_out, a.out_stride, pl->ndm, (int)ntb, part);
   k_dm_stats<<<(pl->ndm + 7) / 8, 256, 0, s>>>(part, (int)ntb, pl->ndm, a.nt_out, a.ave, a.sigma, a.peak, a.frb,

@@ -557,17 +557,17 @@ static int band_launch_t(const BandTables* t, BandParams& k, long long nt_max, c
   const int nb = t->h.nblocks;
   const int nbands = (int)t->h.bands.size();
   // grid y: the most tiles a block has
-  std::vector<unsigned> gy(nbands);
-  for (int bi = 0; bi < nbands; ++bi) {
+  auto tiles = [&](int bi) {
     long long most = 1;
     for (int q = 0; q < nb; ++q) {
       const long long lo = floor_div(t->h.skmin[(size_t)bi * nb + q], NT);
       const long long hi = floor_div(t->h.skmax[(size_t)bi * nb + q] + nt_max - 1, NT);
       most = std::max(most, hi - lo + 1);
     }
-    if (most > 65535) return VFRB_OK;
-    gy[bi] = (unsigned)most;
-  }
+    return most;
+  };
+  for (int bi = 0; bi < nbands; ++bi)
+    if (tiles(bi) > 65535) return VFRB_OK;
   // one limit for every band and plan: launches of other threads set the same
   if (cudaFuncSetAttribute(k_dedisp_band<T, WT, GIVE_UP>, cudaFuncAttributeMaxDynamicSharedMemorySize, kBandSmemMax) !=
       cudaSuccess) {
@@ -586,7 +586,7 @@ static int band_launch_t(const BandTables* t, BandParams& k, long long nt_max, c
     k.first = bi == 0;
     k.last = bi == nbands - 1;
     const size_t smem = band_smem(b.ch, b.lm, t->h.rec_bytes, sizeof(T), WT);
-    const dim3 grid((unsigned)nb, gy[bi], (unsigned)std::max(1, k.njobs));
+    const dim3 grid((unsigned)nb, (unsigned)tiles(bi), (unsigned)std::max(1, k.njobs));
     // A band overlaps the one before it (programmatic dependent launch): its
     // CTAs fill the SMs that the last wave leaves free, and stage and sum their
     // first chunks, before they wait for it to end.  (All CTAs of the band before
