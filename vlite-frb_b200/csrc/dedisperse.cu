@@ -17,8 +17,10 @@
 #include "vfrb_common.cuh"
 
 #include <algorithm>
+#include <atomic>
 #include <cstdint>
 #include <cstdlib>
+#include <mutex>
 #include <vector>
 
 namespace vfrb {
@@ -560,7 +562,8 @@ struct vfrb_ddplan {
   int* d_off = nullptr;
   vfrb::RegGroup reg[3];            // D = 4, 2, 1 when applicable (see ddplan_groups)
   bool group_ok[5] = {};            // [D]: the groups of D trials apply
-  bool groups_built = false;
+  std::atomic<bool> groups_built{false};  // reg is whole and changes no more
+  std::mutex groups_mu;             // of whoever builds it
   int variant[3] = {0, 0, 0};       // chosen variant per storage form (VFRB_DD_*)
   // AUTO runs its own kernels where they apply (launch_auto), else the fastest of
   // the others when they have been timed, else the default
@@ -572,6 +575,7 @@ struct vfrb_ddplan {
 namespace vfrb {
 
 static const RegGroup* find_group(const vfrb_ddplan* pl, int D) {
+  if (!pl->groups_built.load(std::memory_order_acquire)) return nullptr;
   for (const auto& g : pl->reg)
     if (g.D == D) return &g;
   return nullptr;
@@ -1117,6 +1121,15 @@ int ddplan_variant(const vfrb_ddplan* pl, int storage) {
   return resolve_auto(pl, storage);
 }
 
+static void free_group(RegGroup& g) {
+  cudaFree(g.d_gbase);
+  cudaFree(g.d_gpack);
+  cudaFree(g.d_bmin);
+  cudaFree(g.d_bmin16);
+  cudaFree(g.d_gpat);
+  g = RegGroup{};
+}
+
 // Pattern id of the packed in-group differences (8 bits per trial, trial 0
 // first), kPatGeneric when the pattern has no straight-line code.
 static unsigned char pattern_id(int D, unsigned pk) {
@@ -1144,7 +1157,9 @@ static unsigned char pattern_id(int D, unsigned pk) {
   return kPatGeneric;
 }
 
-static int build_group(vfrb_ddplan* p, const int32_t* h_off, int D, int smax_allowed) {
+// the tables of groups of D trials, by copies on cs, in the first free one of reg
+static int build_group(const vfrb_ddplan* p, RegGroup (&reg)[3], const int32_t* h_off, int D, int smax_allowed,
+                       cudaStream_t cs) {
   const int ndm = p->ndm, nchan = p->nchan;
   const int ng = (ndm + D - 1) / D;
   const int DB = kRegWarps * D;
@@ -1194,7 +1209,7 @@ static int build_group(vfrb_ddplan* p, const int32_t* h_off, int D, int smax_all
       span16 = std::max(span16, mx - mn);
     }
   RegGroup* slot = nullptr;
-  for (auto& r : p->reg)
+  for (auto& r : reg)
     if (r.D == 0) {
       slot = &r;
       break;
@@ -1224,18 +1239,15 @@ static int build_group(vfrb_ddplan* p, const int32_t* h_off, int D, int smax_all
             cudaMalloc(&g.d_bmin, bm.size() * sizeof(int)) == cudaSuccess &&
             cudaMalloc(&g.d_bmin16, bm16.size() * sizeof(int)) == cudaSuccess &&
             (!with_pat || cudaMalloc(&g.d_gpat, pt.size()) == cudaSuccess);
-  ok = ok && cudaMemcpy(g.d_gbase, gb.data(), gb.size() * sizeof(int), cudaMemcpyHostToDevice) == cudaSuccess &&
-       cudaMemcpy(g.d_gpack, gp.data(), gp.size() * sizeof(unsigned), cudaMemcpyHostToDevice) == cudaSuccess &&
-       cudaMemcpy(g.d_bmin, bm.data(), bm.size() * sizeof(int), cudaMemcpyHostToDevice) == cudaSuccess &&
-       cudaMemcpy(g.d_bmin16, bm16.data(), bm16.size() * sizeof(int), cudaMemcpyHostToDevice) == cudaSuccess &&
-       (!with_pat || cudaMemcpy(g.d_gpat, pt.data(), pt.size(), cudaMemcpyHostToDevice) == cudaSuccess);
+  auto put = [&](void* d, const auto& v) {
+    return cudaMemcpyAsync(d, v.data(), v.size() * sizeof(v[0]), cudaMemcpyHostToDevice, cs) == cudaSuccess;
+  };
+  ok = ok && put(g.d_gbase, gb) && put(g.d_gpack, gp) && put(g.d_bmin, bm) && put(g.d_bmin16, bm16) &&
+       (!with_pat || put(g.d_gpat, pt));
+  ok = cudaStreamSynchronize(cs) == cudaSuccess && ok;
   if (!ok) {
     cudaGetLastError();
-    cudaFree(g.d_gbase);
-    cudaFree(g.d_gpack);
-    cudaFree(g.d_bmin);
-    cudaFree(g.d_bmin16);
-    cudaFree(g.d_gpat);
+    free_group(g);
     return VFRB_ERR_NOMEM;
   }
   *slot = g;
@@ -1247,23 +1259,47 @@ constexpr int kGroupSmax4 = VFRB_PAT4_SMAX, kGroupSmax2 = VFRB_PAT2_SMAX;
 // Tables of the register-window and pattern kernels.  Where the band kernel
 // applies they are built when a variant is chosen or timed (their tables cost as
 // much to make as the rest of the plan): before any launch that uses them, so
-// that no launch allocates.
+// that no launch allocates.  By one thread, whatever other threads choose or launch
+// meanwhile, and beside any capture: on a stream of its own, in the relaxed mode.
 static int ddplan_groups(vfrb_ddplan* p, const int32_t* h_off) {
-  if (p->groups_built) return VFRB_OK;
+  if (p->groups_built.load(std::memory_order_acquire)) return VFRB_OK;
+  std::lock_guard<std::mutex> lk(p->groups_mu);
+  if (p->groups_built.load(std::memory_order_relaxed)) return VFRB_OK;
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  cudaStream_t cs = nullptr;
+  if (cudaThreadExchangeStreamCaptureMode(&mode) != cudaSuccess) {
+    cudaGetLastError();
+    return VFRB_ERR_CUDA;
+  }
+  if (cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking) != cudaSuccess) {
+    cudaGetLastError();
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    return VFRB_ERR_CUDA;
+  }
+  int st = VFRB_OK;
   std::vector<int32_t> back;
   if (!h_off) {
     back.resize((size_t)p->ndm * p->nchan);
-    if (cudaMemcpy(back.data(), p->d_off, back.size() * sizeof(int32_t), cudaMemcpyDeviceToHost) != cudaSuccess) {
+    if (cudaMemcpyAsync(back.data(), p->d_off, back.size() * sizeof(int32_t), cudaMemcpyDeviceToHost, cs) !=
+            cudaSuccess ||
+        cudaStreamSynchronize(cs) != cudaSuccess) {
       cudaGetLastError();
-      return VFRB_ERR_CUDA;
+      st = VFRB_ERR_CUDA;
     }
     h_off = back.data();
   }
-  int st = VFRB_OK;
-  if (p->group_ok[4]) st = build_group(p, h_off, 4, kGroupSmax4);
-  if (!st && p->group_ok[2]) st = build_group(p, h_off, 2, kGroupSmax2);
-  if (!st && p->group_ok[1]) st = build_group(p, h_off, 1, 0);
-  p->groups_built = st == VFRB_OK;
+  RegGroup reg[3];
+  if (!st && p->group_ok[4]) st = build_group(p, reg, h_off, 4, kGroupSmax4, cs);
+  if (!st && p->group_ok[2]) st = build_group(p, reg, h_off, 2, kGroupSmax2, cs);
+  if (!st && p->group_ok[1]) st = build_group(p, reg, h_off, 1, 0, cs);
+  if (st) {
+    for (auto& g : reg) free_group(g);
+  } else {
+    for (int i = 0; i < 3; ++i) p->reg[i] = reg[i];
+    p->groups_built.store(true, std::memory_order_release);
+  }
+  cudaStreamDestroy(cs);
+  cudaThreadExchangeStreamCaptureMode(&mode);
   return st;
 }
 
@@ -1271,13 +1307,7 @@ int ddplan_destroy(vfrb_ddplan* p) {
   if (!p) return VFRB_OK;
   if (p->d_off) cudaFree(p->d_off);
   band_destroy(p->band);
-  for (auto& g : p->reg) {
-    if (g.d_gbase) cudaFree(g.d_gbase);
-    if (g.d_gpack) cudaFree(g.d_gpack);
-    if (g.d_bmin) cudaFree(g.d_bmin);
-    if (g.d_bmin16) cudaFree(g.d_bmin16);
-    if (g.d_gpat) cudaFree(g.d_gpat);
-  }
+  for (auto& g : p->reg) free_group(g);
   delete p;
   return VFRB_OK;
 }
