@@ -235,11 +235,12 @@ def run_device(vf, frames, storage, steps, warmup, dist, variant=0):
     ms = start.elapsed_time(stop) / steps
     ms = dist_max(dist, ms)
     stage /= steps
+    dd_kernel, dd_launches = pipe.plan.kernel(storage)
     return dict(ms=ms, stage_ms=stage.tolist(), rows=pipe.rows, md=pipe.md, clocks=clk.summary(),
                 stats=pipe.stats, nchan=pipe.L.nchanout,
-                # K1, K2, then seven bands + k_series_part + k_dm_stats, or one pinned kernel + k_dm_stats
-                launches=4 if variant else 11, tune=pipe.tune,
-                variant=pipe.plan.variant(storage) if variant else "auto (band-wise)")
+                # K1, K2, the dedispersion's own, and its statistics
+                launches=2 + dd_launches + (2 if dd_kernel in (vf.DD_BAND, vf.DD_FEW) else 1), tune=pipe.tune,
+                variant={vf.DD_BAND: "auto (band-wise)", vf.DD_FEW: "auto (streaming)"}.get(dd_kernel, dd_kernel))
 
 
 # --------------------------------------------------------------------------- e2e through the plan API

@@ -176,8 +176,9 @@ typedef struct vfrb_ddplan vfrb_ddplan;
 int vfrb_ddplan_create(vfrb_ddplan** plan, const int32_t* h_offsets, int ndm, int nchan);
 int vfrb_ddplan_destroy(vfrb_ddplan* plan);
 int vfrb_ddplan_max_delay(const vfrb_ddplan* plan);
-/* Trials per register group of the fast kernel (4, 2 or 1), 0 when only the
- * staged/direct kernels apply (no reference counterpart; introspection). */
+/* Trials per register group (4, 2 or 1) of the variant that
+ * vfrb_ddplan_variant names for FP32, 0 for the staged/direct kernels (no
+ * reference counterpart; introspection). */
 int vfrb_ddplan_group_size(const vfrb_ddplan* plan);
 
 /* Kernel variants of the dedisperser (no reference counterpart).  AUTO runs
@@ -194,7 +195,16 @@ int vfrb_ddplan_group_size(const vfrb_ddplan* plan);
 #define VFRB_DD_PAT2 7     /* register window, 2 trials, runs of one delay pattern */
 #define VFRB_DD_NVARIANTS 8
 int vfrb_ddplan_set_variant(vfrb_ddplan* plan, int storage, int variant);
+/* The variant chosen; with AUTO the one of the list above that runs calls
+ * which neither of AUTO's own kernels takes. */
 int vfrb_ddplan_variant(const vfrb_ddplan* plan, int storage);
+/* The kernel that a call runs: a variant, or one of AUTO's own.  sigma != 0:
+ * a call with sigma_out.  *launches (may be NULL): its launches without
+ * statistics, which take one more, or two with AUTO's own kernels.  (For rows
+ * whose layout allows 16-byte accesses, and up to 4 million samples.) */
+#define VFRB_DD_BAND 8   /* band-wise: shared partial sums of equally spaced trials */
+#define VFRB_DD_FEW 9    /* streaming: few trials                                   */
+int vfrb_ddplan_kernel(const vfrb_ddplan* plan, int storage, int sigma, int* launches);
 /* The dedispersion kernels' waits for their own copies are bounded; a call
  * whose wait gives up ends by itself and adds 8 to its d_err, and its outputs
  * are not whole.  on != 0: in FP32 calls of the band-wise and the pattern

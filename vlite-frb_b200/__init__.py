@@ -20,6 +20,7 @@ VFRB_OK, VFRB_EOD, VFRB_ERR = 0, 1, 2
 F32, F16, I8 = 0, 1, 2
 DD_AUTO, DD_STAGED, DD_REG1, DD_REG2, DD_REG4, DD_DIRECT, DD_PAT4, DD_PAT2 = 0, 1, 2, 3, 4, 5, 6, 7
 DD_NVARIANTS = 8
+DD_BAND, DD_FEW = 8, 9  # AUTO's own kernels
 
 
 class VfrbError(RuntimeError):
@@ -106,6 +107,7 @@ _lib.vfrb_ddplan_max_delay.argtypes = [C.c_void_p]
 _lib.vfrb_ddplan_group_size.argtypes = [C.c_void_p]
 _lib.vfrb_ddplan_set_variant.argtypes = [C.c_void_p, C.c_int, C.c_int]
 _lib.vfrb_ddplan_variant.argtypes = [C.c_void_p, C.c_int]
+_lib.vfrb_ddplan_kernel.argtypes = [C.c_void_p, C.c_int, C.c_int, C.POINTER(C.c_int)]
 _lib.vfrb_ddplan_set_give_up.argtypes = [C.c_void_p, C.c_int]
 _lib.vfrb_ddplan_autotune.argtypes = [C.c_void_p, C.c_int, C.c_int64, C.c_void_p, C.c_void_p]
 _lib.vfrb_dedisperse_workspace_bytes.restype = C.c_size_t
@@ -258,6 +260,12 @@ class DedispPlan:
 
     def variant(self, storage: int = F32) -> int:
         return int(_lib.vfrb_ddplan_variant(self._p, storage))
+
+    def kernel(self, storage: int = F32, sigma: bool = False):
+        """(kernel, launches) of a call without statistics (vfrb_ddplan_kernel): DD_*, DD_BAND or DD_FEW."""
+        n = C.c_int(0)
+        k = int(_lib.vfrb_ddplan_kernel(self._p, storage, int(sigma), C.byref(n)))
+        return k, n.value
 
     def set_give_up(self, on: bool):
         """The kernels' bounded waits for their own copies give up at once (vfrb_ddplan_set_give_up)."""

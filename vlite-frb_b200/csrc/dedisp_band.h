@@ -12,6 +12,7 @@ struct BandTables;
 // are not close to equally spaced).  VFRB_ERR_NOMEM when device memory runs out.
 int band_create(BandTables** out, const int32_t* h_off, int ndm, int nchan);
 void band_destroy(BandTables* t);
+int band_launches(const BandTables* t);  // of a call
 
 // The dedispersed series of one call (njobs == 0) or of the jobs of a batched
 // launch (grid z = job; the fields of `a` that DdJob holds are ignored).

@@ -851,6 +851,12 @@ static DdKParams dd_params(const vfrb_ddplan* pl, const vfrb_dd_args& a) {
   return k;
 }
 
+// the kernel that AUTO runs by itself, AUTO when it takes a variant's
+static int auto_kernel(const vfrb_ddplan* pl, bool sigma) {
+  if (pl->ndm <= (sigma ? kFewTrialsSigma : kFewTrials)) return VFRB_DD_FEW;
+  return pl->band && !sigma ? VFRB_DD_BAND : VFRB_DD_AUTO;
+}
+
 // samples of a part: 32768 of the streaming kernel's blocks, 16384 band tiles (int8),
 // beside which a band's delays may take the other 49,000 tiles, 12.6 million rows
 constexpr long long kAutoPart = 1LL << 22;
@@ -861,7 +867,8 @@ static int launch_auto(const vfrb_ddplan* pl, const vfrb_dd_args& a, cudaStream_
   *launched = 0;
   const bool want_stats = a.ave || a.sigma || a.peak || a.frb || a.argmax;
   const long long ntb = (a.nt_out + kPartNt - 1) / kPartNt;
-  if (want_stats && ntb * pl->ndm > 0x7fffffffLL) return VFRB_OK;
+  const int kernel = auto_kernel(pl, a.sigma_out != nullptr);
+  if (kernel == VFRB_DD_AUTO || (want_stats && ntb * pl->ndm > 0x7fffffffLL)) return VFRB_OK;
   // The kernels' time blocks are a grid's second dimension, of 65535 at most: longer
   // calls run in parts (a sample's sums do not depend on the cut).
   for (long long t0 = 0; t0 < a.nt_out; t0 += kAutoPart) {
@@ -872,13 +879,13 @@ static int launch_auto(const vfrb_ddplan* pl, const vfrb_dd_args& a, cudaStream_
     b.out += t0;
     if (b.sigma_out) b.sigma_out += t0;
     int st = VFRB_OK, part = 0;
-    if (pl->ndm <= (a.sigma_out ? kFewTrialsSigma : kFewTrials)) {
+    if (kernel == VFRB_DD_FEW) {
       const DdKParams k = dd_params(pl, b);
       if (a.sigma_out) st = few_launch_t<float, true>(pl, k, s, &part);
       else if (a.storage == VFRB_F32) st = few_launch_t<float, false>(pl, k, s, &part);
       else if (a.storage == VFRB_F16) st = few_launch_t<__half, false>(pl, k, s, &part);
       else st = few_launch_t<int8_t, false>(pl, k, s, &part);
-    } else if (pl->band && !a.sigma_out) {
+    } else {
       st = band_launch(pl->band, b, nullptr, 0, pl->give_up, s, &part);
     }
     if (st) return st;
@@ -958,9 +965,9 @@ int launch_dedisperse_jobs(const vfrb_ddplan* pl, int storage, const DdJob* jobs
   *launched = 0;
   if (!pl || njobs < 1 || njobs > kDdMaxJobs || storage < VFRB_F32 || storage > VFRB_F16) return VFRB_ERR_ARG;
   const int v = resolve_auto(pl, storage);
-  const bool band = pl->variant[storage] == VFRB_DD_AUTO && pl->band;
-  // (the streaming kernel has no batched form: the caller launches it per stream)
-  if (pl->variant[storage] == VFRB_DD_AUTO && pl->ndm <= kFewTrials) return VFRB_OK;
+  const int own = pl->variant[storage] == VFRB_DD_AUTO ? auto_kernel(pl, false) : VFRB_DD_AUTO;
+  const bool band = own == VFRB_DD_BAND;
+  if (own == VFRB_DD_FEW) return VFRB_OK;  // no batched form: the caller launches it per stream
   if (!band && v != VFRB_DD_PAT4 && v != VFRB_DD_PAT2) return VFRB_OK;
   vfrb_dd_args a{};
   a.fb = jobs[0].fb;
@@ -1119,6 +1126,15 @@ int ddplan_set_give_up(vfrb_ddplan* pl, int on) {
 int ddplan_variant(const vfrb_ddplan* pl, int storage) {
   if (!pl || storage < VFRB_F32 || storage > VFRB_I8) return -1;
   return resolve_auto(pl, storage);
+}
+
+int ddplan_kernel(const vfrb_ddplan* pl, int storage, bool sigma, int* launches) {
+  if (!pl || storage < VFRB_F32 || storage > VFRB_I8 || (sigma && storage != VFRB_F32)) return -1;
+  const int own = pl->variant[storage] == VFRB_DD_AUTO ? auto_kernel(pl, sigma) : VFRB_DD_AUTO;
+  if (launches) *launches = own == VFRB_DD_BAND ? band_launches(pl->band) : 1;
+  if (own != VFRB_DD_AUTO) return own;
+  const int v = resolve_auto(pl, storage);
+  return sigma && v != VFRB_DD_DIRECT ? VFRB_DD_STAGED : v;
 }
 
 static void free_group(RegGroup& g) {

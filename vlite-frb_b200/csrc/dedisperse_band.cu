@@ -516,6 +516,8 @@ void band_destroy(BandTables* t) {
   delete t;
 }
 
+int band_launches(const BandTables* t) { return (int)t->h.bands.size(); }
+
 int band_create(BandTables** out, const int32_t* off, int ndm, int nchan) {
   *out = nullptr;
   std::unique_ptr<BandTables> t(new BandTables());

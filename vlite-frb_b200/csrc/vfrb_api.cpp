@@ -15,6 +15,7 @@ int ddplan_reg_group(const vfrb_ddplan* p);
 int ddplan_autotune(vfrb_ddplan* pl, int storage, long long nt, float* times, cudaStream_t s);
 int ddplan_set_variant(vfrb_ddplan* pl, int storage, int v);
 int ddplan_variant(const vfrb_ddplan* pl, int storage);
+int ddplan_kernel(const vfrb_ddplan* pl, int storage, bool sigma, int* launches);
 int ddplan_set_give_up(vfrb_ddplan* pl, int on);
 }  // namespace vfrb
 
@@ -150,6 +151,10 @@ int vfrb_ddplan_group_size(const vfrb_ddplan* plan) { return plan ? vfrb::ddplan
 
 int vfrb_ddplan_set_variant(vfrb_ddplan* plan, int storage, int variant) {
   return vfrb::ddplan_set_variant(plan, storage, variant);
+}
+
+int vfrb_ddplan_kernel(const vfrb_ddplan* plan, int storage, int sigma, int* launches) {
+  return vfrb::ddplan_kernel(plan, storage, sigma != 0, launches);
 }
 
 int vfrb_ddplan_set_give_up(vfrb_ddplan* plan, int on) { return vfrb::ddplan_set_give_up(plan, on); }
