@@ -1,0 +1,28 @@
+"""Results at the sizes where a stage call changes its kernel, on both sides of each line,
+against the FP64 oracle."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _rows(rows, nch, seed):
+    return np.random.default_rng(seed).standard_normal((rows, nch)).astype(np.float32) * 2.0 + 5.0
+
+
+@pytest.mark.parametrize("rows,ncol", [(7, 2), (1000, 16), (1023, 1023), (1024, 1024), (1025, 1025), (2048, 1024),
+                                       (2500, 1024), (2500, 1025), (9000, 4096)])
+def test_chan_stats_lines(vf, O, rows, ncol):
+    """Blocks of 1024 rows, all whole, and every other kind.  FP64 sums of values of
+    order 10, stored as float: 1e-6."""
+    import torch
+    nch, nblk = 41, -(-rows // ncol)
+    if rows - (nblk - 1) * ncol == 1:
+        nblk -= 1  # (a last block of one row has no variance)
+    x = _rows(rows, nch, rows + ncol)
+    x[rows // 2, 3] = 1e4
+    a, s, o = vf.chan_stats(torch.from_numpy(np.ascontiguousarray(x.T)).cuda(), rows, ncol, nblk)
+    a_r, s_r, o_r = O.calcstats_chan(x.astype(np.float64), ncol, nblk)
+    assert np.allclose(a.cpu().numpy(), a_r, rtol=1e-6, atol=0)
+    assert np.allclose(s.cpu().numpy(), s_r, rtol=1e-6, atol=1e-9)
+    assert np.array_equal(o.cpu().numpy(), o_r)

@@ -20,13 +20,17 @@ constexpr int kBpFullThreads = 256;  // threads of a channel
 // Channel statistics: the rows of a block are an int, whose largest a last step passes.
 using StatsRow = unsigned;
 
-// f(t) for t = first, first + STEP, ... < nrows
+// f(t) for t = first, first + STEP, ... < nrows; UNROLL 0: unrolled as the compiler likes
 template <int STEP, int UNROLL, typename Row, typename F>
 VFRB_WALK_HD void walk_rows(Row first, Row nrows, F f) {
+  if constexpr (UNROLL == 0) {
+    for (Row t = first; t < nrows; t += STEP) f(t);
+  } else {
 #ifdef __CUDA_ARCH__
 #pragma unroll UNROLL
 #endif
-  for (Row t = first; t < nrows; t += STEP) f(t);
+    for (Row t = first; t < nrows; t += STEP) f(t);
+  }
 }
 
 }  // namespace vfrb
