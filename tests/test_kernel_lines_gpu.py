@@ -26,3 +26,22 @@ def test_chan_stats_lines(vf, O, rows, ncol):
     assert np.allclose(a.cpu().numpy(), a_r, rtol=1e-6, atol=0)
     assert np.allclose(s.cpu().numpy(), s_r, rtol=1e-6, atol=1e-9)
     assert np.array_equal(o.cpu().numpy(), o_r)
+
+
+@pytest.mark.parametrize("rows,ncol,nch", [(6, 2, 70), (446, 223, 300), (448, 224, 300), (300, 223, 64), (700, 224, 65),
+                                           (223, 5000, 257), (224, 5000, 256)])
+def test_chan_sk_lines(vf, O, rows, ncol, nch):
+    """Spectral kurtosis of blocks shorter and longer than a CTA's sets of rows want,
+    ragged last blocks and channel groups: FP64, stored as float.  SK - 1 is a small
+    difference of terms of order 1 times (m nsum + 1) / (m - 1): 1e-6 of the terms."""
+    import torch
+    x = _rows(rows, nch, rows)
+    n = -(-rows // ncol)
+    got = vf.chan_sk(torch.from_numpy(x).cuda(), ncol, n, 20).cpu().numpy()
+    for k in range(n):
+        b = x[k * ncol:(k + 1) * ncol].astype(np.float64)
+        m = len(b)
+        if m == 1:
+            continue
+        f = (m * 20 + 1) / (m - 1)
+        assert np.allclose(got[k], f * (m * (b * b).sum(0) / b.sum(0) ** 2 - 1), rtol=1e-6, atol=1e-12 * f)

@@ -349,18 +349,21 @@ int launch_chan_stats(const vfrb_cs_args& a, cudaStream_t s) {
 // (steady tones) or far above it (bursts); a one-row block gives inf/NaN as
 // M - 1 = 0.  FP64 sums.  The FB is time-major, so a warp reads 32 consecutive
 // channels of a row: 128-byte segments.
-// A CTA takes 64 channels of one block: 16 sets of threads share its rows out
-// (set g rows g, g + 16, ..., eight loads in flight per thread), and the sets'
-// sums are added in order.  (A thread per channel alone gives 175 CTAs of 1024
-// serial loads at 6250 channels x 7 blocks.)
-constexpr int kSkChan = 64, kSkSets = 16;
-__global__ void __launch_bounds__(kSkChan * kSkSets) k_chan_sk(const float* __restrict__ fb, long long row_stride,
-                                                               long long row0, unsigned long long row_mask, int nchan,
-                                                               int nrows, int ncolstatblk, int nstatblks, double nsum,
-                                                               float* __restrict__ sk) {
-  __shared__ double red[2][kSkSets][kSkChan];
-  const int cl = threadIdx.x % kSkChan, g = threadIdx.x / kSkChan;
-  const int c = blockIdx.x * kSkChan + cl;
+// A CTA takes CH channels of one block: SETS sets of threads share its rows out (set g
+// rows g, g + SETS, ..., eight loads in flight per thread), and the sets' sums are added
+// in order.  64 x 16 for blocks of kSkLong rows or more: a thread per channel alone gives
+// 175 CTAs of 1024 serial loads at 6250 channels x 7 blocks (93 -> 39 us).  256 x 1 for
+// shorter ones, which leave most of the sets without a row (3908 channels x 7680 rows,
+// blocks of 64 55 -> 29 us, of 16 172 -> 29 us; at 192 35 against 31, at 256 31 against 35).
+constexpr int kSkLong = 224;
+template <int CH, int SETS>
+__global__ void __launch_bounds__(CH * SETS) k_chan_sk(const float* __restrict__ fb, long long row_stride,
+                                                       long long row0, unsigned long long row_mask, int nchan,
+                                                       int nrows, int ncolstatblk, int nstatblks, double nsum,
+                                                       float* __restrict__ sk) {
+  __shared__ double red[2][SETS][SETS > 1 ? CH : 1];
+  const int cl = threadIdx.x % CH, g = threadIdx.x / CH;
+  const int c = blockIdx.x * CH + cl;
   const int k = blockIdx.y;
   const long long r0 = (long long)ncolstatblk * k;
   const long long r1 = min(r0 + ncolstatblk, (long long)nrows);
@@ -369,10 +372,10 @@ __global__ void __launch_bounds__(kSkChan * kSkSets) k_chan_sk(const float* __re
   double s1 = 0.0, s2 = 0.0;
   long long r = r0 + g;
   constexpr int U = 8;
-  for (; r + (U - 1) * kSkSets < r1; r += U * kSkSets) {
+  for (; r + (U - 1) * SETS < r1; r += U * SETS) {
     float v[U];
 #pragma unroll
-    for (int u = 0; u < U; ++u) v[u] = at(r + u * kSkSets);
+    for (int u = 0; u < U; ++u) v[u] = at(r + u * SETS);
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       const double d = (double)v[u];
@@ -380,16 +383,18 @@ __global__ void __launch_bounds__(kSkChan * kSkSets) k_chan_sk(const float* __re
       s2 += d * d;
     }
   }
-  for (; r < r1; r += kSkSets) {
+  for (; r < r1; r += SETS) {
     const double d = (double)at(r);
     s1 += d;
     s2 += d * d;
   }
-  red[0][g][cl] = s1;
-  red[1][g][cl] = s2;
-  __syncthreads();
+  if constexpr (SETS > 1) {
+    red[0][g][cl] = s1;
+    red[1][g][cl] = s2;
+    __syncthreads();
+  }
   if (g != 0 || c >= nchan) return;
-  for (int q = 1; q < kSkSets; ++q) {
+  for (int q = 1; q < SETS; ++q) {
     s1 += red[0][q][cl];
     s2 += red[1][q][cl];
   }
@@ -405,9 +410,12 @@ int launch_chan_sk_ring(const float* fb_tm, long long row_stride, long long row0
   if (!fb_tm || !sk || nchan <= 0 || nstatblks <= 0 || ncolstatblk <= 1 || nsum < 1 || row_stride < nchan ||
       (long long)nrows - (long long)ncolstatblk * (nstatblks - 1) < 1 || nstatblks > 65535 || row0 < 0)
     return VFRB_ERR_ARG;
-  dim3 grid((unsigned)((nchan + kSkChan - 1) / kSkChan), (unsigned)nstatblks);
-  k_chan_sk<<<grid, kSkChan * kSkSets, 0, s>>>(fb_tm, row_stride, row0, row_mask, nchan, nrows, ncolstatblk, nstatblks,
-                                 (double)nsum, sk);
+  auto run = [&](auto kern, int ch, int threads) {
+    kern<<<dim3((unsigned)((nchan + ch - 1) / ch), (unsigned)nstatblks), threads, 0, s>>>(
+        fb_tm, row_stride, row0, row_mask, nchan, nrows, ncolstatblk, nstatblks, (double)nsum, sk);
+  };
+  if (std::min(ncolstatblk, nrows) >= kSkLong) run(k_chan_sk<64, 16>, 64, 1024);
+  else run(k_chan_sk<256, 1>, 256, 256);
   return cuda_status(cudaGetLastError());
 }
 
