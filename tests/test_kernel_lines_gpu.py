@@ -45,3 +45,25 @@ def test_chan_sk_lines(vf, O, rows, ncol, nch):
             continue
         f = (m * 20 + 1) / (m - 1)
         assert np.allclose(got[k], f * (m * (b * b).sum(0) / b.sum(0) ** 2 - 1), rtol=1e-6, atol=1e-12 * f)
+
+
+@pytest.mark.parametrize("rows", [2, 5, 255, 256, 257, 1024, 1025, 1028, 2047, 2048, 2049, 2052, 6144, 6145, 6148, 8191,
+                                  8192, 8196])
+@pytest.mark.parametrize("row0", [0, 3])
+def test_subtract_bp_full_lines(vf, O, rows, row0):
+    """Whole-block bandpass in registers, in quads and in shared memory, at the edges of
+    each, with the rows aligned or not: one float rounding of the values."""
+    import torch
+    nch = 128
+    x = _rows(rows, nch, rows) - 5.0  # (the reference's first mean divides by the channels)
+    x[rows // 3, 2] += 50.0  # clipped
+    buf = torch.full((nch, (row0 + rows + 7) // 4 * 4), 7.0, device="cuda")
+    buf[:, row0:row0 + rows] = torch.from_numpy(np.ascontiguousarray(x.T)).cuda()
+    vf.subtract_bp_full(buf, nrows=rows, row0=row0)
+    ref = O.subtract_bp_full(x.astype(np.float64))
+    got = buf.cpu().numpy()
+    assert (got[:, :row0] == 7.0).all() and (got[:, row0 + rows:] == 7.0).all()
+    want = ref.T
+    assert np.array_equal(np.isnan(got[:, row0:row0 + rows]), np.isnan(want))
+    ok = ~np.isnan(want)
+    assert np.max(np.abs(got[:, row0:row0 + rows] - want)[ok], initial=0.0) <= 1e-6 * np.abs(x).max()

@@ -44,14 +44,13 @@ __device__ __forceinline__ float clip_lo(double lo) { return __double2float_rd(l
 // ---- whole-block clipped channel mean ------------------------------------------
 // One CTA (256 threads) per channel.  NV > 0: a thread keeps NV rows of the channel
 // in registers, all of their loads in flight at once, in quads of neighbouring rows
-// where these are aligned (VEC).  NV = 0: longer channels, in shared memory (CACHED)
-// or read in every pass.
+// where these are aligned (VEC).  NV = 0: in shared memory (CACHED), or, for channels
+// too long for it, read in every pass.
 //
-// NV = 32 leaves 64 registers a thread, four CTAs per SM; 8192 rows are its limit, and
-// 2048 that of NV = 8, whose loops are short enough for a few hundred rows.  Bound by
-// the FP64 sums and conversions (three per value) and the three reductions.  7680
-// rows x 6250 channels: 144 us with four passes over memory, 102 us through shared
-// memory with 4-byte accesses and every thread dividing, 93 us.
+// NV = 32 leaves 64 registers a thread, four CTAs per SM; 8192 rows are its limit.
+// Bound by the FP64 sums and conversions (three per value) and the three reductions.
+// 7680 rows x 6250 channels: 144 us with four passes over memory, 117 us through shared
+// memory, 100 us in registers and quads; 3071 x 3908 49 -> 39 us, 60 x 3908 20 -> 19 us.
 template <int NV, bool VEC, bool CACHED>
 __global__ void __launch_bounds__(256, NV ? 4 : 1) k_subtract_bp_full(float* __restrict__ fb, long long chan_stride, long long row0,
                                                           unsigned row_mask, int nchan, long long nrows) {
@@ -409,12 +408,16 @@ int launch_subtract_bp_full(float* fb, long long chan_stride, long long row0, un
   if (!rfi_args_ok(fb, chan_stride, row0, row_mask, nchan, nrows)) return VFRB_ERR_ARG;
   const bool vec = rfi_quads(fb, chan_stride, row0, row_mask) && (nrows & 3) == 0;
   auto run = [&](auto kern, size_t smem) {
-    kern<<<nchan, 256, smem, s>>>(fb, chan_stride, row0, row_mask, nchan, nrows);
+    kern<<<nchan, kBpFullThreads, smem, s>>>(fb, chan_stride, row0, row_mask, nchan, nrows);
   };
-  if (nrows <= 8 * 256) {
+  // Registers where their number is nearly the rows', and by quads for the larger one;
+  // else shared memory, which has no test for each row in its loops.  3908 channels, us,
+  // registers against shared memory: 60 rows 25 / 19, 1024 25 / 25, 2000 33 (27 in quads)
+  // / 35, 3071 70 / 39, 5000 (quads) 55 / 49, 7680 88 (66) / 78.
+  if (nrows > 4 * 256 && nrows <= 8 * 256) {
     vec ? run(k_subtract_bp_full<8, true, false>, 0) : run(k_subtract_bp_full<8, false, false>, 0);
-  } else if (nrows <= 32 * 256) {
-    vec ? run(k_subtract_bp_full<32, true, false>, 0) : run(k_subtract_bp_full<32, false, false>, 0);
+  } else if (vec && nrows > 24 * 256 && nrows <= 32 * 256) {
+    run(k_subtract_bp_full<32, true, false>, 0);
   } else if (nrows * 4 <= kRfiSmem) {
     if (const int st = rfi_smem(k_subtract_bp_full<0, false, true>)) return st;
     run(k_subtract_bp_full<0, false, true>, (size_t)nrows * 4);
