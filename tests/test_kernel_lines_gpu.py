@@ -67,3 +67,21 @@ def test_subtract_bp_full_lines(vf, O, rows, row0):
     assert np.array_equal(np.isnan(got[:, row0:row0 + rows]), np.isnan(want))
     ok = ~np.isnan(want)
     assert np.max(np.abs(got[:, row0:row0 + rows] - want)[ok], initial=0.0) <= 1e-6 * np.abs(x).max()
+
+
+@pytest.mark.parametrize("nch,rows", [(2, 167), (2, 168), (3, 5000), (64, 5375), (64, 5376), (192, 16127), (192, 16128),
+                                      (193, 16300), (193, 2**19)])
+@pytest.mark.parametrize("row0", [0, 5])
+def test_subtract_zero_lines(vf, O, nch, rows, row0):
+    """Zero-DM with a thread per row for many rows beside the channels, and with clusters:
+    one float rounding of the values."""
+    import torch
+    x = _rows(rows, nch, rows + nch)
+    x[rows // 3] += 20.0  # a broadband row
+    x[rows // 2, 1] += 500.0  # clipped
+    buf = torch.full((nch, (row0 + rows + 7) // 4 * 4), 7.0, device="cuda")
+    buf[:, row0:row0 + rows] = torch.from_numpy(np.ascontiguousarray(x.T)).cuda()
+    vf.subtract_zero(buf, nrows=rows, row0=row0)
+    got = buf.cpu().numpy()
+    assert (got[:, :row0] == 7.0).all() and (got[:, row0 + rows:] == 7.0).all()
+    assert np.max(np.abs(got[:, row0:row0 + rows] - O.subtract_zero(x).T)) <= 1e-6 * np.abs(x).max()

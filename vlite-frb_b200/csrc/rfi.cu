@@ -341,9 +341,10 @@ __global__ void __launch_bounds__(kZeroThreads, 1024 / kZeroThreads)
   cluster.barrier_wait();  // no CTA leaves while another may read its sums
 }
 
-// More channels than fit in shared memory: one thread per row; a warp covers 32
-// consecutive rows, so every channel's load is one 128-byte segment
-__global__ void __launch_bounds__(256) k_subtract_zero_wide(float* __restrict__ fb, long long chan_stride, long long row0,
+// More channels than fit in shared memory, or many rows for them (launch_subtract_zero):
+// one thread per row; a warp covers 32 consecutive rows, so every channel's load is one
+// 128-byte segment
+__global__ void __launch_bounds__(256) k_subtract_zero_rows(float* __restrict__ fb, long long chan_stride, long long row0,
                                                             unsigned row_mask, int nchan, long long nrows) {
   const long long t = (long long)blockIdx.x * 256 + threadIdx.x;
   if (t >= nrows) return;
@@ -434,7 +435,14 @@ int launch_subtract_zero(float* fb, long long chan_stride, long long row0, unsig
   int k = 1;
   while (k < 8 && slice(k) > kZeroSlice) k *= 2;
   const long long smem = slice(k);
-  if (smem <= kRfiSmem) {
+  // A thread per row reads its channels four times: from the caches where 256 rows of
+  // all channels fit there, and with enough rows for every SM; with very many rows its
+  // plain loads keep more in flight than the clusters' short lives.  us, thread per row
+  // against clusters: 64 channels x 1024 rows 10.3 / 8.8, 7680 10.3 / 14.4, 2^17 29 / 153;
+  // 192 x 7680 45 / 16, 2^14 23 / 29, 2^17 102 / 195; 256 x 2^15 64 / 53, 2^17 245 / 207,
+  // 2^19 581 / 865; 1024 x 2^17 969 / 386, 2^19 2312 / 2327, 2^20 4632 / 5744.
+  const bool rows = (nchan <= 192 && nrows >= 84LL * nchan) || (nchan <= 1024 && nrows >= 1LL << 19);
+  if (smem <= kRfiSmem && !rows) {
     const long long nb = (nrows + kZeroRows - 1) / kZeroRows * k;
     if (nb > 0x7fffffffLL) return VFRB_ERR_UNSUPPORTED;
     const bool vec = rfi_quads(fb, chan_stride, row0, row_mask);
@@ -460,7 +468,7 @@ int launch_subtract_zero(float* fb, long long chan_stride, long long row0, unsig
   } else {
     const long long nb = (nrows + 255) / 256;
     if (nb > 0x7fffffffLL) return VFRB_ERR_UNSUPPORTED;
-    k_subtract_zero_wide<<<(unsigned)nb, 256, 0, s>>>(fb, chan_stride, row0, row_mask, nchan, nrows);
+    k_subtract_zero_rows<<<(unsigned)nb, 256, 0, s>>>(fb, chan_stride, row0, row_mask, nchan, nrows);
   }
   return cuda_status(cudaGetLastError());
 }
