@@ -85,3 +85,12 @@ def test_subtract_zero_lines(vf, O, nch, rows, row0):
     got = buf.cpu().numpy()
     assert (got[:, :row0] == 7.0).all() and (got[:, row0 + rows:] == 7.0).all()
     assert np.max(np.abs(got[:, row0:row0 + rows] - O.subtract_zero(x).T)) <= 1e-6 * np.abs(x).max()
+
+
+@pytest.mark.parametrize("nch,rows", [(1, 1), (2, 33), (12, 1000), (13, 1000), (12, 32 * 65535), (12, 32 * 65535 + 1), (64, 64),
+                                      (65, 129)])
+def test_transpose_lines(vf, nch, rows):
+    """Small and large tiles, and the rows that a grid of the small ones has: equal bits."""
+    import torch
+    x = torch.randn((nch, rows + 3), device="cuda")
+    assert torch.equal(vf.fb_to_time_major(x, nrows=rows, row0=2), x[:, 2:2 + rows].t())
