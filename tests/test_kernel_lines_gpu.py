@@ -94,3 +94,18 @@ def test_transpose_lines(vf, nch, rows):
     import torch
     x = torch.randn((nch, rows + 3), device="cuda")
     assert torch.equal(vf.fb_to_time_major(x, nrows=rows, row0=2), x[:, 2:2 + rows].t())
+
+
+@pytest.mark.parametrize("nt", [1, 2, 100, 191, 192, 193])
+@pytest.mark.parametrize("width", [1, 2, 64])
+def test_boxcar_short_series(vf, O, nt, width):
+    """Series around the shortest that go through tiles, with sums that are exact."""
+    import torch
+    x = np.round(np.random.default_rng(nt).standard_normal((33, nt)) * 64).astype(np.float32) / 64
+    x[5, nt // 2:nt // 2 + 7] += 3.0
+    x[0] = 0.5  # equal samples: the smaller width, then the earlier start
+    ave, sig = x.mean(axis=1).astype(np.float32), np.maximum(x.std(axis=1), 0.25).astype(np.float32)
+    best, start, w = O.boxcar_best(x, ave, sig, width)
+    snr, s0, w0 = vf.boxcar(torch.from_numpy(x).cuda(), torch.from_numpy(ave).cuda(), torch.from_numpy(sig).cuda(), width)
+    assert np.array_equal(w0.cpu().numpy(), w) and np.array_equal(s0.cpu().numpy(), start)
+    assert np.allclose(snr.cpu().numpy(), best, rtol=1e-6, atol=1e-9)
