@@ -1281,20 +1281,24 @@ static int ddplan_groups(vfrb_ddplan* p, const int32_t* h_off) {
   if (p->groups_built.load(std::memory_order_acquire)) return VFRB_OK;
   std::lock_guard<std::mutex> lk(p->groups_mu);
   if (p->groups_built.load(std::memory_order_relaxed)) return VFRB_OK;
+  // (a plan being made, h_off given, is nobody else's yet: the default stream will do)
   cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
   cudaStream_t cs = nullptr;
-  if (cudaThreadExchangeStreamCaptureMode(&mode) != cudaSuccess) {
-    cudaGetLastError();
-    return VFRB_ERR_CUDA;
-  }
-  if (cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking) != cudaSuccess) {
-    cudaGetLastError();
-    cudaThreadExchangeStreamCaptureMode(&mode);
-    return VFRB_ERR_CUDA;
+  const bool beside = !h_off;
+  if (beside) {
+    if (cudaThreadExchangeStreamCaptureMode(&mode) != cudaSuccess) {
+      cudaGetLastError();
+      return VFRB_ERR_CUDA;
+    }
+    if (cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking) != cudaSuccess) {
+      cudaGetLastError();
+      cudaThreadExchangeStreamCaptureMode(&mode);
+      return VFRB_ERR_CUDA;
+    }
   }
   int st = VFRB_OK;
   std::vector<int32_t> back;
-  if (!h_off) {
+  if (beside) {
     back.resize((size_t)p->ndm * p->nchan);
     if (cudaMemcpyAsync(back.data(), p->d_off, back.size() * sizeof(int32_t), cudaMemcpyDeviceToHost, cs) !=
             cudaSuccess ||
@@ -1314,8 +1318,10 @@ static int ddplan_groups(vfrb_ddplan* p, const int32_t* h_off) {
     for (int i = 0; i < 3; ++i) p->reg[i] = reg[i];
     p->groups_built.store(true, std::memory_order_release);
   }
-  cudaStreamDestroy(cs);
-  cudaThreadExchangeStreamCaptureMode(&mode);
+  if (beside) {
+    cudaStreamDestroy(cs);
+    cudaThreadExchangeStreamCaptureMode(&mode);
+  }
   return st;
 }
 
