@@ -476,11 +476,13 @@ int64_t vfrb_plan_device_bytes(const vfrb_plan* plan);
  * another stream must be complete (that stream synchronised) before the
  * call.  `bytes` may be reused as soon as the call returns.
  * Pageable host memory goes through two staging buffers: 16 frames each from
- * the stream's opening, and page-locked for longer runs (up to 41 MB each) in
- * the first two pushes that bring one -- some ms each, once; where that fails
- * the small ones serve on, in smaller copies.  Page-locked and device memory
- * need none of them. */
+ * the stream's opening; the first longer runs page-lock larger ones (up to 41
+ * MB and 40 ms each, once per stream; where that fails the small ones serve on,
+ * in smaller copies).  vfrb_stream_stage does it ahead, for callers that push
+ * pageable memory and want no such push: VFRB_ERR_NOMEM when it failed.
+ * Page-locked and device memory need none of this. */
 int vfrb_push_frames(vfrb_plan* plan, int stream, const uint8_t* bytes, size_t nbytes);
+int vfrb_stream_stage(vfrb_plan* plan, int stream);
 
 /* Streams opened and closed while others run (serving).  vfrb_stream_open
  * admits one more stream if its device bytes fit the budget (device_bytes,

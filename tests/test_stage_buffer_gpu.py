@@ -12,11 +12,15 @@ def test_pageable_pushes_of_growing_size(vf):
     buf = synth.make_vdif(synth.StreamSpec(duration=2.0, seed=5, pulses=[synth.Pulse(0.7, 6.0, 2.0, 40.0)]))
     raw = np.ascontiguousarray(buf.numpy())
 
-    def run(pieces):
+    def run(pieces, stage=False):
         plan = vf.Plan(np.arange(0, 20.5, 0.5, dtype=np.float32), nave=2, muoslowfreq=384.0, mode=vf.MODE_STREAM,
                        outputs=vf.OUT_DEDISP, chunk_seconds=0.5)
+        if stage:
+            plan.stage_stream(0)
         for p in pieces:
             plan.push(0, p)
+            if stage:
+                plan.stage_stream(0)  # (again: nothing to do)
         plan.push(0, None)
         res = plan.drain()
         plan.close()
@@ -32,3 +36,14 @@ def test_pageable_pushes_of_growing_size(vf):
     assert len(pieces) > len(sizes)
     got = run(pieces)
     assert got.shape == want.shape and np.array_equal(got, want)
+    assert np.array_equal(run(pieces, stage=True), want)
+
+
+def test_staging_ahead_refuses_other_streams(vf):
+    plan = vf.Plan(np.arange(0, 2.0, 0.5, dtype=np.float32), nave=2, muoslowfreq=384.0, mode=vf.MODE_STREAM,
+                   outputs=vf.OUT_DEDISP, chunk_seconds=0.5)
+    plan.stage_stream(0)
+    for s in (-1, 1):
+        with pytest.raises(vf.VfrbError):
+            plan.stage_stream(s)
+    plan.close()

@@ -428,6 +428,7 @@ _lib.vfrb_push_frames.argtypes = [C.c_void_p, C.c_int, C.c_void_p, C.c_size_t]
 _lib.vfrb_poll.argtypes = [C.c_void_p, C.POINTER(Result), C.c_int]
 _lib.vfrb_stream_open.argtypes = [C.c_void_p, C.POINTER(C.c_int)]
 _lib.vfrb_stream_close.argtypes = [C.c_void_p, C.c_int]
+_lib.vfrb_stream_stage.argtypes = [C.c_void_p, C.c_int]
 _lib.vfrb_stream_log.restype = C.c_char_p
 _lib.vfrb_stream_log.argtypes = [C.c_void_p, C.c_int]
 
@@ -484,6 +485,10 @@ class Plan:
             return False
         _check(st, "vfrb_stream_close")
         return True
+
+    def stage_stream(self, stream: int):
+        """Page-lock the stream's staging buffers for pageable input now (vfrb_stream_stage)."""
+        _check(_lib.vfrb_stream_stage(self._h, stream), "vfrb_stream_stage")
 
     def push(self, stream: int, data):
         """data: bytes / numpy uint8 / torch uint8 tensor -- CPU (pinned or not)

@@ -996,6 +996,17 @@ int64_t oldest_ref(const StreamSt* s) {
   return o;
 }
 
+// Frames of the next batch of pageable input that staging buffer k takes.  Page-locking
+// the buffers (41 MB each, about 40 ms) was most of a stream's opening: they hold
+// kStageFew frames then (a frame that straddles pushes comes alone), and grow when such
+// input first brings more, or when vfrb_stream_stage asks.
+size_t stage_frames(StreamSt* s, int k, size_t want) {
+  return stage_room(s->stage[k], want, s->stage_frames, [&](size_t frames) {
+    uint8_t* q = nullptr;
+    return hmalloc(s->res, &q, frames * kFrameLen) == VFRB_OK ? q : nullptr;
+  });
+}
+
 // Copy `nf` whole frames to the ring, queue their headers, advance.
 int feed_frames(vfrb_plan* pl, StreamSt* s, const uint8_t* in, int64_t nf, MemKind kind) {
   const Range nvtx_range("vfrb feed frames");
@@ -1008,14 +1019,7 @@ int feed_frames(vfrb_plan* pl, StreamSt* s, const uint8_t* in, int64_t nf, MemKi
   size_t pitch = kFrameLen;  // of the headers the reader reads
   for (int64_t done = 0; done < nf;) {
     int64_t nb = std::min(batch_max, nf - done);
-    // page-locking the staging buffers (up to 41 MB each) was most of a stream's
-    // opening: they hold kStageFew frames then (a frame that straddles pushes comes
-    // alone), and grow when pageable input first brings more
-    if (!pinned && !device)
-      nb = (int64_t)stage_room(s->stage[s->stage_i], (size_t)nb, s->stage_frames, [&](size_t frames) {
-        uint8_t* q = nullptr;
-        return hmalloc(s->res, &q, frames * kFrameLen) == VFRB_OK ? q : nullptr;
-      });
+    if (!pinned && !device) nb = (int64_t)stage_frames(s, s->stage_i, (size_t)nb);
     const uint8_t* src = in + done * kFrameLen;  // host bytes, or device bytes (device input)
     // frames about to be overwritten must have been consumed by launched work
     if (oldest_ref(s) < s->frames_in + nb - s->ring_frames) {
@@ -1437,6 +1441,16 @@ int vfrb_stream_open(vfrb_plan* pl, int* stream) {
   }
   *stream = id;
   return VFRB_OK;
+}
+
+int vfrb_stream_stage(vfrb_plan* pl, int stream) {
+  if (!pl || stream < 0 || stream >= (int)pl->st.size() || !pl->st[stream]) return VFRB_ERR_ARG;
+  StreamSt* s = pl->st[stream].get();
+  if (cudaSetDevice(pl->P.device) != cudaSuccess) return VFRB_ERR_CUDA;
+  int st = VFRB_OK;
+  for (int k = 0; k < kStageBufs; ++k)
+    if (stage_frames(s, k, s->stage_frames) < s->stage_frames) st = VFRB_ERR_NOMEM;
+  return st;
 }
 
 int vfrb_stream_close(vfrb_plan* pl, int stream) {
