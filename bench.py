@@ -766,8 +766,11 @@ def main():
     k1_bytes = data_s * (2 * 25600 * 5032 + nch * (1.0 / (NAVE * 12500 / 128e6)) * 4)
     # K1 FFT work at the usual real-FFT count: 2.5 N log2 N per 12500-sample transform
     k1_flop = data_s * 2 * (128e6 / 12500) * 2.5 * 12500 * math.log2(12500)
-    roofline = {"bound": "fp32_add", "achieved": adds_per_s / 1e12, "peak": fp32_peak_adds / 1e12,
+    roofline = {"bound": "fp32_add (brute-force sums)", "achieved": adds_per_s / 1e12, "peak": fp32_peak_adds / 1e12,
                 "unit": "Tadd/s", "frac": adds_per_s / fp32_peak_adds, "traffic": traffic,
+                "note": "trial-sample-channel sums per second; the band-wise kernel shares partial sums and executes "
+                        "about a quarter as many additions, with no pipe full (shared memory 56%, issue 59%, FMA 25%: "
+                        "profiles/dedisperse_band_16s.md)",
                 "kernel": "dedisperse (K3)",
                 "peak_source": f"{nsm} SMs x 128 FP32 lanes x {sm_mhz:g} MHz (MEASURED_PEAKS.json has no FP32 "
                                f"figure)",

@@ -622,11 +622,18 @@ static int dd_launch_t(const vfrb_ddplan* pl, const vfrb_dd_args& a, DdKParams& 
 }
 
 // Most trials that the streaming kernel takes.  By the trials alone, so that the
-// order of the sums does not change with the number of samples.  Against the band
-// kernel (3908 channels, ms): 16 trials 0.04 / 0.10 / 0.57 against 0.74 / 0.78 /
-// 0.78 at 300 / 2000 / 18,000 samples, 32 trials 0.06 / 0.15 / 1.05 against 0.71 /
-// 0.74 / 0.75.  Sigma form against the staged kernel: 64 trials 0.08 / 0.27 / 2.11
-// against 1.39 / 1.43 / 2.16; two trials x 18,000 (the tool's case) 5.38 -> 0.11.
+// order of the sums does not change with the number of samples.  Streaming against the
+// band kernel, 3908 channels (NAVE 4), trials 2 DM apart (45 bands), ms: 16 trials 0.04 /
+// 0.15 / 0.51 / 1.78 against 0.68 / 0.71 / 0.72 / 1.74 at 300 / 4096 / 16,384 / 61,440
+// samples, 32 trials 0.05 / 0.27 / 0.98 / 3.51 against 0.69 / 0.71 / 0.73 / 1.76, 64
+// trials 0.07 / 0.51 / 1.91 / 6.97 against 0.71 / 0.73 / 1.03 / 3.19.  Trials 0.5 DM apart
+// (12 bands): 17 trials 0.04 / 0.15 / 0.54 / 1.91 against 0.21 / 0.21 / 0.26 / 0.69, 64
+// trials 0.07 / 0.49 / 1.90 / 6.96 against 0.21 / 0.21 / 0.40 / 1.30.  So where the lines
+// cross depends on the spacing and on the samples: up to 64 trials, calls of a thousand
+// samples or less would be faster streamed, and long calls of 16 trials band-wise (the
+// pattern kernel takes 1.26 ms at 16 x 61,440, streaming 1.78, the band kernel 0.86 with
+// trials 0.7 DM apart).  Sigma form against the staged kernel: 64 trials 0.08 / 0.27 /
+// 2.11 against 1.39 / 1.43 / 2.16; two trials x 18,000 (the tool's case) 5.38 -> 0.11.
 constexpr int kFewTrials = 16;
 constexpr int kFewTrialsSigma = 64;
 
@@ -1062,10 +1069,11 @@ int ddplan_autotune(vfrb_ddplan* pl, int storage, long long nt, float* times, cu
   }
   float best = 1e30f;
   int bestv = VFRB_DD_STAGED;
-  // AUTO's own kernels are kept wherever they apply, not timed: they were the
-  // fastest at every size tried (1 to 2048 trials, 300 to 18,000 samples, 1.4
-  // times the best of the others and more), and plans made side by side, whose
-  // timings disturb each other, then sum in the same order.
+  // AUTO's own kernels are kept wherever they apply, not timed: against the best of the
+  // variants they took 0.05 to 0.96 of the time at 1 to 2048 trials, 300 to 61,440 samples
+  // (but 1.4 of it for 16 trials x 61,440: see kFewTrials, which chooses between the
+  // two), and plans made side by side, whose timings disturb each other, then sum in the
+  // same order.
   int own = 0;
   if (launch_auto(pl, a, s, &own) != VFRB_OK) own = 0;
   if (times) times[VFRB_DD_AUTO] = -1.f;
