@@ -21,8 +21,8 @@
 // for a plain sum.  At 2048 trials x 6250 channels x 16384 samples the loads keep
 // the shared-memory pipe 57% busy; the rest is latency (dependent branches of the
 // staircases and load latency, four warps per scheduler).  13.5 ms (pattern
-// kernel) -> 6.55 ms; 2048 x 1024 in FP16 1.50 -> 0.74 ms; 201 trials x 5145
-// samples 1.65 -> 0.59 ms, in int8 2.37 (staged kernel) -> 0.84 ms.  Longer runs
+// kernel) -> 6.53 ms; 2048 x 1024 in FP16 1.50 -> 0.74 ms; 201 trials x 5145
+// samples 1.65 -> 0.59 ms, in int8 2.37 (staged kernel) -> 0.83 ms.  Longer runs
 // per lane with fewer warps have fewer loads and instructions per sum but were no
 // faster: TT 11 with 12 warps 7.0 ms, TT 17 with 8 warps 8.5 ms; nor were more
 // warps with shorter runs, TT 7 x 20 warps 7.3 ms.  Two 8-warp CTAs per SM hold
